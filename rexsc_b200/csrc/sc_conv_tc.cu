@@ -1,32 +1,45 @@
-// SC conv forward on the 5th-generation tensor cores (tcgen05, int8 operands, int32 accumulators in TMEM).
+// SC conv forward on the 5th-generation tensor cores (tcgen05, 4-bit operands, fp32 accumulators in TMEM).
 //
 // Per time slot t the count that OR-n saturates is a plain contraction of 0/1 values,
 //     count_t[pixel][sign, co] = sum_{tap, c} a_t[pixel + tap][c] * w_t[sign, co][tap, c],
 // and only min(count_t, n) is non-linear -- it is applied to the finished accumulator of every slot:
 //     out[pixel][sign, co] = sum_t min(count_t, n)            (sc_device.cu:127-151 of the reference).
-// So every slot is one int8 GEMM, M = output-pixel candidates (TMEM lanes, 128 per MMA), N = 128 (64 output
-// channels x {positive, negative} weight stream), K = taps x channels, issued as tcgen05.mma.kind::i8 M128 N128 K32.
+// So every slot is one GEMM with M = 128 rows (64 output channels x {positive, negative} weight stream, the TMEM
+// lanes), N = output-pixel candidates, K = taps x channels, issued as tcgen05.mma.kind::mxf4 M128 N160 K64.
 //
-// Rows.  The M dimension runs over the "origin grid": per image Ho x Wo candidates (i, j), candidate (i, j) being
+// Why 4-bit floats.  0 and the powers of two that the operands use (0.5, 1, 2) are exact e2m1 numbers, every block
+// scale is 1, a coincidence contributes exactly 1.0 and fp32 accumulators count exactly to 2^24: the result is the
+// integer count.  Against the int8 kind the same channels take half the operand bytes and half the MMA time, and
+// expanding 32 bits into 32 operands takes 5 logic instructions instead of 17.
+//
+// Why the weights are the TMEM operand.  The MMA reads its M operand from tensor memory and its N operand from shared
+// memory; with both in shared memory (128 x 128 tiles) operand reads alone fill the shared-memory pipe (8 KB per 64
+// clk).  The pixels have to stay in shared memory, because a filter tap is the same buffer at another start row; the
+// weights have no such need, are expanded straight from registers into TMEM columns, and leave 64 B/clk of operand
+// reads.
+//
+// Columns.  The N dimension runs over the "origin grid": per image Ho x Wo candidates (i, j), candidate (i, j) being
 // the padded-input pixel (i*stride_h, j*stride_w), i.e. the top-left tap of output pixel (i, j) when i < OH and
-// j < OW (other rows are computed and dropped; they are the padding of the grid, a few percent).  A CTA owns 256
-// consecutive candidates.
+// j < OW (other candidates are computed and dropped; they are the padding of the grid, a few percent).  A tile is 320
+// consecutive candidates, two MMA column blocks ("units") of 160.
 //
-// Operands are generated in shared memory from bit planes (one bit per element and slot, 32 channels per word):
-//   A_t  the slot's activation bits of the tile's patch as 16-byte K-columns [16-channel column][patch row][16 B]
-//        (unswizzled K-major, rows 16 bytes apart).  The patch is kept as one plane per stride residue
-//        (kh % stride_h, kw % stride_w); inside a plane, row r holds the pixel of that residue that belongs to
-//        candidate o0 + r.  The operand of filter tap (kh, kw) is then the SAME buffer with its start address moved
-//        to plane(kh % sh, kw % sw) + (kh / sh) * Wo + kw / sw rows: no im2col, for any stride.
-//   B_t  the slot's weight bits, [tap][16-channel column][128 rows][16 B].
-// Operand bytes are 0 or a power of two (see kTcMaskA), the accumulators hold 8 * count.
+// Operands are generated from bit planes (one bit per element and slot, 32 channels per word):
+//   pixels   the slot's activation bits of the tile's patch as 16-byte K-columns [32-channel word][patch row][16 B]
+//            (unswizzled K-major, rows 16 bytes apart).  The patch is kept as one plane per stride residue
+//            (kh % stride_h, kw % stride_w); inside a plane, row r holds the pixel of that residue that belongs to
+//            candidate o0 + r.  The operand of filter tap (kh, kw) is then the SAME buffer with its start address moved
+//            to plane(kh % sh, kw % sw) + (kh / sh) * Wo + kw / sw rows: no im2col, for any stride.
+//   weights  the slot's weight bits, TMEM columns [tap][32-channel word][4 columns of 8 nibbles].
+//
+// Tensor memory (512 columns): two accumulator units of 160, two operand buffers of up to 72, 16 columns of block
+// scales (all 1, the same columns serve both operands).
 //
 // One persistent CTA per SM walks its tiles as a single pipeline (a tile's first loads and its store overlap the
-// neighbouring tiles' MMAs): 16 warps expand operands and fold counts, 2 warps issue MMAs (one per 128-row block; a single
-// thread cannot keep the tensor core busy with 128-column MMAs).  A pipeline step is one slot x one chunk of 32 or
-// 64 channels.  Operand buffers and accumulators are double-buffered and every dependence is an mbarrier phase:
-// while the tensor core works through step i, the expanding warps write the operands of step i+1, fold the slot
-// that finished, and already hold the bit words of step i+2 in registers.
+// neighbouring tiles' MMAs): eight warps fold counts, four expand operands, one issues the MMAs, unit 0 then unit 1 of
+// every step.  A pipeline step is one slot x one chunk of 64 channels (1x1 filters: up to 256).  Operand buffers are
+// double-buffered, a unit's accumulators are folded while the other unit is computed, and every dependence is an
+// mbarrier phase: while the tensor core works through step i, the folding warps are on the unit that finished and
+// the expanding warps write the operands of step i+1.
 // Every wait is bounded; on a time-out the CTA reports through the status word, frees its TMEM and returns.
 #include "common.cuh"
 #include <stdlib.h>
@@ -36,23 +49,40 @@ namespace rexsc {
 
 namespace {
 
-constexpr int kTcWorkers = 512;             // threads that expand operands and fold counts
-constexpr int kTcThreads = kTcWorkers + 64; // + two warps that only issue MMAs, one per 128-row block
-constexpr int kTcM = 256;          // candidates per CTA: two MMA row blocks that share one weight operand
-constexpr int kTcSub = 128;        // rows of one MMA (TMEM lanes)
+constexpr int kTcFoldWarps = 16;            // warps that fold finished accumulators into running sums, eight per unit
+constexpr int kTcExpandWarps = 8;           // warps that expand operands, two per TMEM lane quarter
+constexpr int kTcIssueWarp = kTcFoldWarps + kTcExpandWarps; // issues the MMAs
+constexpr int kTcLoadWarp = kTcIssueWarp + 1;               // copies the weight bit words into shared memory
+constexpr int kTcThreads = (kTcFoldWarps + kTcExpandWarps + 4) * 32; // whole warpgroups: two warps idle
+// Registers per thread: 896 threads are launched with 72, which the warpgroups share out again by what they need (the
+// folding warps hold 40 sum registers and 48 counts).
+constexpr int kTcRegsLaunch = 72, kTcRegsFold = 96, kTcRegsExpand = 40, kTcRegsIssuer = 32;
+static_assert(kTcFoldWarps * 32 * kTcRegsFold + kTcExpandWarps * 32 * kTcRegsExpand + 128 * kTcRegsIssuer <= kTcThreads * kTcRegsLaunch,
+              "more registers than the block has");
+constexpr int kTcMaxDepth = 4;              // pipeline steps whose bit words are in shared memory or on their way
+constexpr int kTcBars = 9 + 2 * kTcMaxDepth;
+constexpr int kTcUnit = 160;       // candidates of one MMA (its N)
+constexpr int kTcM = 2 * kTcUnit;  // candidates per tile: two units that share one weight operand
+constexpr int kTcCols = kTcUnit / 2; // accumulator columns of its unit that one warp folds
 constexpr int kTcCout = 64;        // output channels per CTA
-constexpr int kTcN = 2 * kTcCout;  // MMA N: positive block [0,64), negative block [64,128)
+constexpr int kTcN = 2 * kTcCout;  // weight rows (MMA M, TMEM lanes): positive block [0,64), negative block [64,128)
 constexpr int kTcMaxTaps = 9;      // filter taps whose weight operand is staged at once
-constexpr int kTcMaxARows = 3;     // patch rows per expanding thread (all residue planes together)
-constexpr int kTcMaxBWords = 5;    // weight words per expanding thread and step
-constexpr int kTcPrefetch = 4;     // pipeline steps between the L2 prefetch of patch bits and their use
+constexpr int kTcMaxARows = 8;     // patch rows per expanding thread (all residue planes together)
+constexpr int kTcWordCols = 4;     // TMEM columns of one 32-channel weight word (8 nibbles per column)
+constexpr int kTcMaxWords = 18;    // weight words per row and step: the operand buffers' TMEM columns / kTcWordCols
+constexpr uint32_t kTcColA = 2 * kTcUnit;                                   // first column of the weight buffers
+constexpr uint32_t kTcColSf = kTcColA + 2 * kTcMaxWords * kTcWordCols;      // first column of the block scales
+static_assert(kTcColSf + 16 <= 512, "tensor memory has 512 columns");
+constexpr int kTcStageCols = 32;   // candidates that pass through a warp's store staging at a time
+constexpr int kTcStagePitch = kTcStageCols / 2 + 1; // words per row of a warp's store staging: odd, so rows change banks
 constexpr uint32_t kTcWaitLimit = 1u << 18; // try_wait attempts before a wait gives up (each may sleep kTcSuspendNs)
 constexpr uint32_t kTcSuspendNs = 4000;    // a waiting warp sleeps in the barrier unit instead of spinning on issue slots
 
 struct TcArgs {
     int OH, OW, KHW, Co, CW;
-    int KWc;         // 32-channel words per pipeline step: 2, or 1 when shared memory is short
+    int KWc;         // 32-channel words per pipeline step (even: one MMA takes two)
     int CK;          // pipeline steps per slot = ceil(CW / KWc)
+    int depth;       // steps of bit words kept in shared memory: kTcMaxDepth, or 2 when it is short
     int nrh, nrw, Wq, Hrows, Wrow; // stored pixel grid (see tap_offset in common.cuh)
     int Ho, Wo;      // origin grid of one image
     int shift;       // candidates by which the patch starts BEFORE the tile's first candidate: 0, or Wo + 1 on the
@@ -63,7 +93,7 @@ struct TcArgs {
     long long total_o; // candidates = N * Ho * Wo
     int tiles_x;       // candidate tiles = ceil(total_o / kTcM)
     int total_tiles;   // tiles_x * (64-channel output chunks); tile index = chunk * tiles_x + x
-    int out_vec;       // both output pointers are 16-byte aligned: rows may be stored as 128-bit vectors
+    int out_al4;       // both output pointers are 4-byte aligned: two channels of a pixel may be stored at once
     int balanced;      // 0: a CTA walks whole tiles blockIdx.x, + gridDim.x, ...
                        // 1: the (tile, time slot) pairs, in that order, are cut into gridDim.x equal runs, one per CTA.
                        //    A tile that two or more CTAs share is zeroed before the launch (zero_shared_tiles_kernel)
@@ -73,7 +103,7 @@ struct TcArgs {
                        //    channel runs): the host clears the whole outputs and every tile adds 16-bit values.
     long long NHWp;
     int out_nhwc;
-    int descale_each; // 1: running sums would overflow 16 bits in accumulator units, so every slot is descaled
+    int wide;        // 1: running sums (or the OR-n limit) exceed what fp16 counts exactly, so they are kept as integers
     int tap_off[kTcMaxTaps]; // patch-row offset of every tap (kernel parameters are warp-uniform by construction)
 };
 
@@ -134,46 +164,23 @@ __device__ __forceinline__ bool tc_wait(uint32_t bar, uint32_t parity)
     return false;
 }
 
-// Operand bytes are not 0/1.  Expanding bit i of a nibble to byte i costs one byte-replicate (PRMT) and one AND when
-// the byte keeps its bit where it was: patch bytes are 0 or 2^i (mask 0x08040201).  The weight bit planes store each
-// nibble bit-reversed and use mask 0x01020408, so their bytes are 0 or 2^(3-i); every coincidence contributes
-// 2^i * 2^(3-i) = 8 and the accumulators hold 8 * count.
-constexpr uint32_t kTcMaskA = 0x08040201u, kTcMaskW = 0x01020408u;
-constexpr int kTcScaleLog2 = 3;
-constexpr uint32_t kDescaleMask = (0xffffu >> kTcScaleLog2) * 0x00010001u; // after a packed 16-bit shift right
-
-// 32 bits -> two groups of 16 operand bytes (bits 0..15 and 16..31; byte i <- bit i)
-template <uint32_t MASK>
-__device__ __forceinline__ void spread32(uint32_t h, uint4 &lo16, uint4 &hi16)
+// 32 bits -> 32 e2m1 operands (16 bytes).  A bit expands by masking where it stands: bits 0, 1, 2 of a nibble are the
+// numbers 0.5, 1 and 2, bit 3 (the sign) is moved down to 2 first.  The weight bit planes store every nibble
+// bit-reversed, so that their numbers are 2, 1, 0.5 and 0.5: every coincidence contributes exactly 1.  Both operands
+// thereby permute the channels of a word in the same way, which a sum does not notice.
+__device__ __forceinline__ uint4 spread_pixels(uint32_t h)
 {
-    const uint32_t g = h >> 4; // high nibbles moved into the low half of each byte
-    lo16.x = __byte_perm(h, 0, 0x0000) & MASK;
-    lo16.y = __byte_perm(g, 0, 0x0000) & MASK;
-    lo16.z = __byte_perm(h, 0, 0x1111) & MASK;
-    lo16.w = __byte_perm(g, 0, 0x1111) & MASK;
-    hi16.x = __byte_perm(h, 0, 0x2222) & MASK;
-    hi16.y = __byte_perm(g, 0, 0x2222) & MASK;
-    hi16.z = __byte_perm(h, 0, 0x3333) & MASK;
-    hi16.w = __byte_perm(g, 0, 0x3333) & MASK;
+    return make_uint4(h & 0x11111111u, h & 0x22222222u, h & 0x44444444u, (h >> 1) & 0x44444444u);
+}
+__device__ __forceinline__ uint4 spread_weights(uint32_t h)
+{
+    const uint32_t g = h >> 1;
+    return make_uint4(g & 0x44444444u, g & 0x22222222u, g & 0x11111111u, h & 0x11111111u);
 }
 
-#define REXSC_TMEM_LD32(arr, taddr)                                                                                   \
+#define REXSC_TMEM_LD16(arr, taddr)                                                                                   \
     asm volatile(                                                                                                     \
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "                                                                     \
-        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "                                     \
-        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"                     \
-        : "=r"(arr[0]), "=r"(arr[1]), "=r"(arr[2]), "=r"(arr[3]), "=r"(arr[4]), "=r"(arr[5]), "=r"(arr[6]),           \
-          "=r"(arr[7]), "=r"(arr[8]), "=r"(arr[9]), "=r"(arr[10]), "=r"(arr[11]), "=r"(arr[12]), "=r"(arr[13]),       \
-          "=r"(arr[14]), "=r"(arr[15]), "=r"(arr[16]), "=r"(arr[17]), "=r"(arr[18]), "=r"(arr[19]), "=r"(arr[20]),    \
-          "=r"(arr[21]), "=r"(arr[22]), "=r"(arr[23]), "=r"(arr[24]), "=r"(arr[25]), "=r"(arr[26]), "=r"(arr[27]),    \
-          "=r"(arr[28]), "=r"(arr[29]), "=r"(arr[30]), "=r"(arr[31])                                                  \
-        : "r"(taddr)                                                                                                  \
-        : "memory")
-
-// 32 TMEM columns as 16 registers: the low 16 bits of two adjacent columns per register
-#define REXSC_TMEM_LD16_PACKED(arr, taddr)                                                                            \
-    asm volatile(                                                                                                     \
-        "tcgen05.ld.sync.aligned.32x32b.x16.pack::16b.b32 "                                                           \
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "                                                                     \
         "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"                              \
         : "=r"(arr[0]), "=r"(arr[1]), "=r"(arr[2]), "=r"(arr[3]), "=r"(arr[4]), "=r"(arr[5]), "=r"(arr[6]),           \
           "=r"(arr[7]), "=r"(arr[8]), "=r"(arr[9]), "=r"(arr[10]), "=r"(arr[11]), "=r"(arr[12]), "=r"(arr[13]),       \
@@ -181,13 +188,31 @@ __device__ __forceinline__ void spread32(uint32_t h, uint4 &lo16, uint4 &hi16)
         : "r"(taddr)                                                                                                  \
         : "memory")
 
+// wait for the thread's TMEM reads; the registers are operands so that nothing that uses them can move ahead of it
+#define REXSC_TMEM_WAIT16(arr)                                                                                        \
+    asm volatile("tcgen05.wait::ld.sync.aligned;"                                                                     \
+        : "+r"(arr[0]), "+r"(arr[1]), "+r"(arr[2]), "+r"(arr[3]), "+r"(arr[4]), "+r"(arr[5]), "+r"(arr[6]),           \
+          "+r"(arr[7]), "+r"(arr[8]), "+r"(arr[9]), "+r"(arr[10]), "+r"(arr[11]), "+r"(arr[12]), "+r"(arr[13]),       \
+          "+r"(arr[14]), "+r"(arr[15])                                                                                \
+        :: "memory")
 // KHW_T: taps known at compile time (9, 1) or 0 for any tap count up to kTcMaxTaps
-// KWC:   32-channel words per pipeline step (TcArgs::KWc);  RA: patch rows per expanding thread (1 .. kTcMaxARows)
+// KWC:   32-channel words per pipeline step (TcArgs::KWc; above 4 only with KHW_T == 1)
+// RA:    patch rows per expanding thread (1 .. kTcMaxARows)
+//
+// What bounds it, and the split of the warps.  The MMAs of a step take 18 x 83 clk on a 3x3 layer; everything else has
+// to fit beside them.  Folding costs three instructions per two counts (convert, minimum, add; the first two on the ALU,
+// at half rate) and expanding five per 32 operands, so the instruction count decides, and with it what every warp
+// repeats per step: addresses, waits, hand-overs.  Measured on 64 -> 64 channels, 3x3, 56x56, 32 slots, batch 256 (whole
+// call; tensor pipe busy): int8 operands, both in shared memory, 16 warps on both jobs 1.13 ms (80 % of an int8 pipe of
+// half the rate); 4-bit with 16 such warps 1.32 ms (43 %); 8 folding + 4 expanding warps 0.95 ms; 8 + 8 with the weight
+// words brought in by bulk copies 1.01 ms (48 %; the folding warps waited for five TMEM reads per unit, one after the
+// other); 16 folding warps, eight per unit, + 8 expanding: 0.84 ms.  512 -> 512 channels, 7x7: 1.19 -> 0.69 ms (87 %).
 template <int KHW_T, int KWC, int RA>
 __global__ void __launch_bounds__(kTcThreads, 1)
 sc_conv_tc_kernel(TcArgs a, const uint32_t *__restrict__ Ab, const uint32_t *__restrict__ Wb,
                   int16_t *__restrict__ out_pos, int16_t *__restrict__ out_neg, int *__restrict__ status, int gate)
 {
+    static_assert(KWC % 2 == 0 && (KWC <= 4 || KHW_T == 1), "an MMA takes two words");
     extern __shared__ __align__(16) uint8_t smem_raw[];
     // One of a pair of launches, of which the expand stage's verdict on the activation borders (status word 1: 0 =
     // the compact planes are valid) picks one: +1 runs on valid compact planes only, -1 on the standard planes that
@@ -195,17 +220,17 @@ sc_conv_tc_kernel(TcArgs a, const uint32_t *__restrict__ Ab, const uint32_t *__r
     if (gate != 0 && (gate > 0) == (status[1] != 0)) return;
     uint8_t *smem = smem_raw + ((128u - (saddr(smem_raw) & 127u)) & 127u);
     const int KHW = KHW_T ? KHW_T : a.KHW;
-    const uint32_t a_bytes = 2u * (uint32_t)KWC * (uint32_t)a.rows_a * 16u; // [2*KWc columns][rows_a][16]
-    const uint32_t b_bytes = (uint32_t)KHW * 2u * (uint32_t)KWC * kTcN * 16u; // [KHW][2*KWc columns][128][16]
-    auto a_buf = [&](int buf) { return smem + (uint32_t)buf * a_bytes; };
-    auto b_buf = [&](int buf) { return smem + 2 * a_bytes + (uint32_t)buf * b_bytes; };
-    uint64_t *bars = reinterpret_cast<uint64_t *>(smem + 2 * a_bytes + 2 * b_bytes);
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 8);
+    const uint32_t a_bytes = (uint32_t)KWC * (uint32_t)a.rows_a * 16u; // [KWC words][rows_a][16]
+    uint32_t *stage_all = reinterpret_cast<uint32_t *>(smem + 2 * a_bytes); // [fold warp][32 rows][kTcStagePitch]
+    uint32_t *w_ring = stage_all + kTcFoldWarps * 32 * kTcStagePitch;       // [depth][tap][KWC][kTcN] weight bit words
+    uint32_t *p_ring = w_ring + a.depth * (KHW * KWC * kTcN);               // [depth][RA][KWC][256] patch bit words
+    uint64_t *bars = reinterpret_cast<uint64_t *>(p_ring + a.depth * (RA * KWC * kTcExpandWarps * 32));
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + kTcBars);
 
     const int tid = threadIdx.x, lane = tid & 31;
     // the shuffle tells the compiler what it cannot see: the warp index is the same in every lane
     const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
-    // Persistent CTA: it runs its tiles as ONE pipeline, so a tile's first loads / expansion and its last epilogue /
+    // Persistent CTA: it runs its tiles as ONE pipeline, so a tile's first loads / expansion and its last fold /
     // store overlap the neighbouring tiles' MMAs.  Its k-th tile is tile first_tile + k * tile_stride, of which it
     // computes time slots [slot_lo(k), slot_hi(k)): all of them, except in the first and last tile of a balanced run.
     // (The run is needed at tile switches only: it lives in shared memory, not in registers.)
@@ -220,24 +245,35 @@ sc_conv_tc_kernel(TcArgs a, const uint32_t *__restrict__ Ab, const uint32_t *__r
         o0 = (long long)(L - nc * a.tiles_x) * kTcM;         // first candidate of the tile
     };
 
-    // mbarriers (index = operand buffer or accumulator buffer):
-    //   full[b]   operands of a step are in shared memory           (one arrival per expanding warp)
-    //   empty[b]  the MMAs that read operand buffer b have completed  (one commit per issuing warp); after the last
-    //             chunk of a slot this also says that the slot's counts are complete in their accumulator buffer
-    //   tfree[t]  accumulator buffer t has been folded                (one arrival per expanding warp)
-    //   drain     every MMA of an issuing warp has completed          (one commit per issuing warp, at its exit)
-    uint64_t *bar_full = bars, *bar_empty = bars + 2, *bar_tfree = bars + 4, *bar_drain = bars + 6;
+    // mbarriers (index = operand buffer b or unit u):
+    //   full[b]   operands of a step are written                         (one arrival per expanding warp)
+    //   empty[b]  the MMAs that read operand buffer b have completed     (one commit per step)
+    //   done[u]   unit u's counts of a slot are complete                 (one commit per slot)
+    //   tfree[u]  unit u's accumulators have been read                   (one arrival per folding warp)
+    //   drain     every MMA has completed                                (one commit, at the issuing warp's exit)
+    //   wfull[d]  the weight bit words of a step are in ring entry d     (bytes of the copies)
+    //   wfree[d]  they have been expanded                                (one arrival per expanding warp)
+    uint64_t *bar_full = bars, *bar_empty = bars + 2, *bar_tfree = bars + 4, *bar_done = bars + 6, *bar_drain = bars + 8;
+    uint64_t *bar_wfull = bars + 9, *bar_wfree = bars + 9 + kTcMaxDepth;
     if (tid == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(saddr(bar_drain)), "r"(kTcM / kTcSub) : "memory");
+        auto init = [](uint64_t *bar, uint32_t count) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(saddr(bar)), "r"(count) : "memory");
+        };
+        init(bar_drain, 1u);
         for (int b = 0; b < 2; b++) {
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(saddr(&bar_full[b])), "r"(kTcWorkers / 32) : "memory");
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(saddr(&bar_empty[b])), "r"(kTcM / kTcSub) : "memory");
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(saddr(&bar_tfree[b])), "r"(kTcWorkers / 32) : "memory");
+            init(&bar_full[b], kTcExpandWarps);
+            init(&bar_empty[b], 1u);
+            init(&bar_done[b], 1u);
+            init(&bar_tfree[b], kTcFoldWarps / 2);
+        }
+        for (int d = 0; d < kTcMaxDepth; d++) {
+            init(&bar_wfull[d], 1u);
+            init(&bar_wfree[d], kTcExpandWarps);
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 0) {
-        // two accumulator buffers of 2 row blocks x 128 columns: the whole tensor memory of the SM.  The allocation
+        // the whole tensor memory of the SM.  The allocation
         // blocks until all 512 columns are free, so this kernel assumes it is the only user of tensor memory on its
         // SM: its > 113 KB of dynamic shared memory keeps a second CTA of itself away, but a kernel of ANOTHER stream
         // that holds tensor memory (the FXP conv of this library, a vendor GEMM) would make the allocation wait for
@@ -250,210 +286,23 @@ sc_conv_tc_kernel(TcArgs a, const uint32_t *__restrict__ Ab, const uint32_t *__r
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = *tmem_slot;
-    const int my_tiles = run.tiles;
-
-    // instruction descriptor: int32 accumulators, signed int8 operands, both K-major, N = 128, M = 128
-    const uint32_t idesc = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kTcN >> 3) << 17) | ((uint32_t)(kTcSub >> 4) << 24);
-    const uint32_t a_lbo = (uint32_t)a.rows_a * 16, b_lbo = kTcN * 16;
-    const int wrow_words = KHW * a.CW;                 // weight words per row and slot
-
-    // running sums: this thread owns row block (warp/4)%2, TMEM lane 32*(warp%4)+lane and 64 columns (warp/8 = 0:
-    // positive block, 1: negative block), two 16-bit sums per register as the packed TMEM load delivers them
-    uint32_t acc[32];
-#pragma unroll
-    for (int j = 0; j < 32; j++) acc[j] = 0u;
-    const uint32_t my_tcol = ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(((warp >> 2) & 1) * kTcN + (warp >> 3) * 64);
-    const uint32_t n2 = ((uint32_t)a.n_or << kTcScaleLog2) * 0x00010001u; // the clamp, in accumulator units, twice
-
-    // ---- what an expanding thread loads and writes -------------------------------------------------------------
-    // Bit words of a step are fetched into registers two steps before their MMAs so that L2 latency is hidden; the
-    // loads walk the steps in order, so the step-dependent part of every address is a running pointer.
-    //   weights: item e = tid + 512*i, row = e & 127, (tap, word) = e >> 7  -> wbits[i]
-    //   patch:   row g = tid + 512*r of the residue planes                  -> abits[r][word]
-    // weight words per thread and step: ceil(taps * words / 4) when the tap count is known at compile time
-    constexpr int kMyB = KHW_T ? (KHW_T * KWC + 3) / 4 : kTcMaxBWords;
-    uint32_t wbits[kMyB], abits[RA][KWC];
-    const int w_row = tid & (kTcN - 1), w_rest0 = tid >> 7;               // (tap, word) index of item 0
-    const int w_half = KWC == 2 ? (w_rest0 & 1) : 0;
-    const int w_tap0 = KWC == 2 ? (w_rest0 >> 1) : w_rest0;
-    const int w_items = KHW * KWC;                                      // (tap, word) pairs per step
-    const size_t w_item_stride = (size_t)(4 / KWC) * a.CW * kTcN;       // item i -> i + 1: 4 pairs further
-    const uint32_t *w_ptr = Wb, *a_plane = Ab, *pf_plane = Ab;
-    uint32_t a_off[RA]; // stored-grid position of the thread's patch rows, ~0u: outside the tensor
-    const bool pf_on = (a.CW % KWC) == 0;                                // planes are then visited in storage order
-    int ld_ck = 0, ld_left = 0, ld_tile = -1;
-    // point the loads at tile k of this CTA: slot 0, chunk 0
-    auto load_tile = [&](int k) {
-        long long o0;
-        int nc;
-        tile_origin(k, o0, nc);
-        const int slot0 = slot_lo(k);                                      // first slot of the tile
-        ld_tile = k;
-        ld_ck = 0;
-        ld_left = (slot_hi(k) - slot0) * a.CK;
-        w_ptr = Wb + ((size_t)nc * a.slots + slot0) * kTcN * wrow_words + ((size_t)w_tap0 * a.CW + w_half) * kTcN + w_row;
-        a_plane = Ab + (size_t)slot0 * a.CW * a.NHWp;                       // bit plane of the first slot, word 0
-        pf_plane = a_plane + (size_t)kTcPrefetch * KWC * a.NHWp;
-#pragma unroll
-        for (int r = 0; r < RA; r++) {
-            const int g = tid + kTcWorkers * r;
-            a_off[r] = ~0u;
-            if (g < a.rows_a) {
-                const int plane = g / a.Mh, q = g - plane * a.Mh;
-                // candidate indices fit 31 bits (checked on the host); rows before the first stored pixel wrap around
-                // to large values and are zero like the rows behind the last one
-                const uint32_t o = (uint32_t)o0 + (uint32_t)q - (uint32_t)a.shift;
-                if (o < (uint32_t)a.total_o) {
-                    const uint32_t t = o / (uint32_t)a.Wo, j = o - t * (uint32_t)a.Wo;
-                    const uint32_t n = t / (uint32_t)a.Ho, i = t - n * (uint32_t)a.Ho;
-                    const int rh = plane / a.nrw, rw = plane - rh * a.nrw;
-                    a_off[r] = (n * (uint32_t)a.Hrows + i * (uint32_t)a.nrh + (uint32_t)rh) * (uint32_t)a.Wrow +
-                               (uint32_t)(rw * a.Wq) + j; // < NHWp < 2^32
-                }
-            }
-        }
-    };
-    auto load_bits = [&]() {
-        const int words_left = a.CW - ld_ck * KWC; // words of this chunk that exist
-#pragma unroll
-        for (int i = 0; i < kMyB; i++) {
-            const bool ok = w_rest0 + 4 * i < w_items && w_half < words_left;
-            wbits[i] = ok ? __ldg(w_ptr + i * w_item_stride) : 0u;
-        }
-#pragma unroll
-        for (int r = 0; r < RA; r++) {
-            abits[r][0] = a_off[r] != ~0u ? __ldg(a_plane + a_off[r]) : 0u;
-            if (KWC == 2) abits[r][KWC - 1] = (a_off[r] != ~0u && words_left > 1) ? __ldg(a_plane + a.NHWp + a_off[r]) : 0u;
-        }
-        // the patch bits stream from HBM: pull the lines of a later step into L2 (one lane per 128-byte line)
-        if (pf_on && lane == 0 && ld_left > kTcPrefetch) {
-#pragma unroll
-            for (int r = 0; r < RA; r++)
-                if (a_off[r] != ~0u) {
-                    asm volatile("prefetch.global.L2 [%0];" ::"l"(pf_plane + a_off[r]));
-                    if (KWC == 2) asm volatile("prefetch.global.L2 [%0];" ::"l"(pf_plane + a.NHWp + a_off[r]));
-                }
-        }
-        // advance to the next step: next chunk of the slot, or chunk 0 of the next slot
-        ld_left--;
-        if (++ld_ck == a.CK) {
-            ld_ck = 0;
-            w_ptr += ((size_t)wrow_words - (size_t)KWC * (a.CK - 1)) * kTcN;
-            a_plane += (size_t)(a.CW - KWC * (a.CK - 1)) * a.NHWp;
-        } else {
-            w_ptr += (size_t)KWC * kTcN;
-            a_plane += (size_t)KWC * a.NHWp;
-        }
-        pf_plane += (size_t)KWC * a.NHWp;
-        if (ld_left == 0 && ld_tile + 1 < my_tiles) load_tile(ld_tile + 1); // the next call fetches the next tile
-    };
-    // per-thread shared-memory offsets of the expansion targets (buffer 0)
-    const uint32_t b_dst0 = (uint32_t)(((w_tap0 * 2 * KWC + 2 * w_half) * kTcN + w_row) * 16);
-    const uint32_t a_kcol = (uint32_t)a.rows_a * 16;
-    auto expand_bits = [&](int buf) {
-        uint8_t *b_s = b_buf(buf) + b_dst0, *a_s = a_buf(buf) + (uint32_t)tid * 16;
-#pragma unroll
-        for (int i = 0; i < kMyB; i++) {
-            if (w_rest0 + 4 * i < w_items) {
-                uint8_t *dst = b_s + i * (8 * kTcN * 16); // 4 (tap, word) pairs = 8 K-columns further
-                uint4 lo16, hi16;
-                spread32<kTcMaskW>(wbits[i], lo16, hi16);
-                *reinterpret_cast<uint4 *>(dst) = lo16;
-                *reinterpret_cast<uint4 *>(dst + kTcN * 16) = hi16;
-            }
-        }
-#pragma unroll
-        for (int r = 0; r < RA; r++) {
-            if (tid + kTcWorkers * r < a.rows_a) {
-                uint8_t *dst = a_s + r * (kTcWorkers * 16);
-                uint4 lo16, hi16;
-                spread32<kTcMaskA>(abits[r][0], lo16, hi16);
-                *reinterpret_cast<uint4 *>(dst) = lo16;
-                *reinterpret_cast<uint4 *>(dst + a_kcol) = hi16;
-                if (KWC == 2) {
-                    spread32<kTcMaskA>(abits[r][KWC - 1], lo16, hi16);
-                    *reinterpret_cast<uint4 *>(dst + 2 * a_kcol) = lo16;
-                    *reinterpret_cast<uint4 *>(dst + 3 * a_kcol) = hi16;
-                }
-            }
-        }
-    };
-    // count -> min(count, n) -> running sums, for the slot whose accumulators sit in TMEM buffer `tbuf`
-    auto slot_epilogue = [&](int tbuf) {
-        const uint32_t taddr = tmem_base + my_tcol + (uint32_t)(tbuf * 2 * kTcN);
-        uint32_t v0[16], v1[16];
-        REXSC_TMEM_LD16_PACKED(v0, taddr);
-        REXSC_TMEM_LD16_PACKED(v1, taddr + 32u);
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        if (!a.descale_each) {
-#pragma unroll
-            for (int j = 0; j < 16; j++) {
-                acc[j] += __vminu2(v0[j], n2);
-                acc[16 + j] += __vminu2(v1[j], n2);
-            }
-        } else {
-#pragma unroll
-            for (int j = 0; j < 16; j++) {
-                acc[j] += (__vminu2(v0[j], n2) >> kTcScaleLog2) & kDescaleMask;
-                acc[16 + j] += (__vminu2(v1[j], n2) >> kTcScaleLog2) & kDescaleMask;
-            }
-        }
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    };
-    // One thread issues the MMAs of one 128-row block.  A single thread gets one 128-column MMA through about every
-    // 128 clocks, half of what the tensor core can take, so the two row blocks are issued from two warps.  The
-    // issuing warps share their schedulers with the expanding warps, so the loop is kept to a few instructions per
-    // MMA: fully unrolled over taps, per-tap operand offsets in registers, descriptors patched in their low word
-    // (the start-address field counts 16-byte units, i.e. operand rows, from bit 0; no carry leaves the field
-    // because shared memory ends below 256 KB).
-    const int my_sub = warp - kTcWorkers / 32;
-    uint32_t a_tap[kTcMaxTaps];
-#pragma unroll
-    for (int tap = 0; tap < kTcMaxTaps; tap++)
-        a_tap[tap] = (my_sub >= 0 && tap < KHW) ? (uint32_t)(my_sub * kTcSub + a.tap_off[tap]) : 0u;
-    const uint64_t da_proto = desc_interleaved(saddr(a_buf(0)), a_lbo), db_proto = desc_interleaved(saddr(b_buf(0)), b_lbo);
-    const uint32_t da_hi = (uint32_t)(da_proto >> 32), db_hi = (uint32_t)(db_proto >> 32);
-    const uint32_t a_kk = 2u * (uint32_t)a.rows_a;             // rows between the 32-channel words of a chunk
-    const uint32_t b_tap = 2u * (uint32_t)KWC * kTcN;        // rows between taps of the weight operand
-    auto issue_mmas = [&](int step, int s, int ck) {
-        const int buf = step & 1;
-        const uint32_t da_lo = (uint32_t)da_proto + (uint32_t)buf * (a_bytes >> 4);
-        const uint32_t db_lo = (uint32_t)db_proto + (uint32_t)buf * (b_bytes >> 4);
-        const uint32_t d_addr = tmem_base + (uint32_t)((s & 1) * 2 * kTcN + my_sub * kTcN);
-        const bool two = KWC == 2 && ck * 2 + 1 < a.CW; // a second 32-channel word in this chunk
-        const uint32_t first_acc = ck > 0 ? 1u : 0u;
-#pragma unroll
-        for (int tap = 0; tap < (KHW_T ? KHW_T : kTcMaxTaps); tap++) {
-            if (KHW_T || tap < a.KHW) {
-#pragma unroll
-                for (int kk = 0; kk < 2; kk++) {
-                    if (kk == 1 && !two) break;
-                    const uint32_t alo = da_lo + a_tap[tap] + (kk ? a_kk : 0u);
-                    const uint32_t blo = db_lo + (uint32_t)tap * b_tap + (uint32_t)(2 * kk * kTcN);
-                    const uint32_t accumulate = (tap > 0 || kk > 0) ? 1u : first_acc;
-                    asm volatile(
-                        "{\n\t.reg .pred p, e;\n\t.reg .b64 da, db;\n\t"
-                        "mov.b64 da, {%1, %2};\n\t"
-                        "mov.b64 db, {%3, %4};\n\t"
-                        "setp.ne.b32 p, %6, 0;\n\t"
-                        "elect.sync _|e, 0xffffffff;\n\t"
-                        "@e tcgen05.mma.cta_group::1.kind::i8 [%0], da, db, %5, {%7, %7, %7, %7}, p;\n\t}"
-                        ::"r"(d_addr), "r"(alo), "r"(da_hi), "r"(blo), "r"(db_hi), "r"(idesc), "r"(accumulate), "r"(0u)
-                        : "memory");
-                }
-            }
-        }
-        // the commits arrive on their barriers when every MMA issued so far by this warp has completed
-        asm volatile("{\n\t.reg .pred e;\n\telect.sync _|e, 0xffffffff;\n\t"
-                     "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(saddr(&bar_empty[buf]))
-                     : "memory");
-    };
-
-    bool failed = false;
+    const uint32_t lane_quarter = (uint32_t)((warp & 3) * 32) << 16; // the TMEM lanes this warp can access
+    if (warp < 4) {
+        // block scales: 2^0 (biased exponent 127) in every byte, whatever row or block an MMA reads from them
+        const uint32_t one = 0x7f7f7f7fu;
+        asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
+                     "{%1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1};" ::"r"(tmem_base + kTcColSf + lane_quarter),
+                     "r"(one) : "memory");
+        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const int total_steps = run.slots * a.CK; // pipeline steps of this CTA; slots are numbered through all of its tiles
+    bool failed = false;
     // The warps run unsynchronised; every dependence is an mbarrier phase.  Phase parities: barrier index b is used
-    // by steps (or slots) b, b + 2, ...; its k-th completion has parity k & 1.  A timed-out wait ends the warp's
-    // loop; the warps that depend on it time out in turn, so everybody reaches the end of the kernel.
+    // by steps b, b + 2, ... (done, tfree: by every slot); its k-th completion has parity k & 1.  A timed-out wait ends
+    // the warp's loop; the warps that depend on it time out in turn, so everybody reaches the end of the kernel.
     auto wait_on = [&](uint64_t *bar, int k) {
         const bool ok = tc_wait(saddr(bar), (uint32_t)(k & 1));
         return __all_sync(0xffffffffu, ok) != 0;
@@ -462,119 +311,387 @@ sc_conv_tc_kernel(TcArgs a, const uint32_t *__restrict__ Ab, const uint32_t *__r
         __syncwarp();
         if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(saddr(bar)) : "memory");
     };
-    // running sums -> int16 outputs of the tile whose last slot has just been folded; a row is one candidate of the
-    // origin grid, it is an output pixel iff i < OH and j < OW
-    auto store_tile = [&](int k) {
-        long long o0;
-        int nc;
-        tile_origin(k, o0, nc);
-        const bool shared_tile = slot_hi(k) - slot_lo(k) < a.slots; // other CTAs hold the tile's other time slots
-        if (!a.descale_each) {
+
+    // one step further in a ring of a.depth entries; `round` counts the passes through it
+    auto ring_next = [&](int &d, int &round) {
+        if (++d == a.depth) { d = 0; round++; }
+    };
+
+    if (warp >= kTcIssueWarp) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kTcRegsIssuer));
+    if (warp == kTcIssueWarp) {
+        // ---- MMA-issuing warp: operands ready -> accumulator free -> issue -> commit ----
+        // The loop is kept to a few instructions per MMA: fully unrolled over taps, per-tap operand offsets in
+        // registers, descriptors patched in their low word (the start-address field counts 16-byte units, i.e. operand
+        // rows, from bit 0; no carry leaves the field because shared memory ends below 256 KB).
+        // instruction descriptor: e2m1 operands (both K-major), ue8m0 block scales, N = 160, M = 128
+        const uint32_t idesc = (1u << 7) | (1u << 10) | ((uint32_t)(kTcUnit >> 3) << 17) | (1u << 23) | ((uint32_t)(kTcN >> 4) << 24);
+        uint32_t p_tap[kTcMaxTaps];
 #pragma unroll
-            for (int j = 0; j < 32; j++) acc[j] = (acc[j] >> kTcScaleLog2) & kDescaleMask;
-        }
-        const uint32_t o = (uint32_t)o0 + (uint32_t)(((warp >> 2) & 1) * kTcSub + (warp & 3) * 32 + lane);
-        if (o < (uint32_t)a.total_o) {
-            const uint32_t t = o / (uint32_t)a.Wo, n = t / (uint32_t)a.Ho;
-            const int ow = (int)(o - t * (uint32_t)a.Wo), oh = (int)(t - n * (uint32_t)a.Ho);
-            if (ow < a.OW && oh < a.OH) {
-                const int co0 = nc * kTcCout;
-                const size_t ohw = (size_t)a.OH * a.OW;
-                const size_t m = ((size_t)n * a.OH + oh) * a.OW + ow;
-                int16_t *dst = (warp >> 3) ? out_neg : out_pos;
-                if (a.balanced == 2) {
-                    // Any layout: EVERY tile of the launch adds its sums into outputs that the host cleared, one
-                    // 16-bit value per 32-bit atomic add on the word that holds it (no carry leaves the value's half:
-                    // the complete sums fit 16 bits; the word's other half gets + 0).  All accesses to these words are
-                    // atomic adds, so neighbours stored by other CTAs cannot be lost.
-                    const size_t e0 = a.out_nhwc ? m * a.Co + co0 : ((size_t)n * a.Co + co0) * ohw + (size_t)oh * a.OW + ow;
-                    const size_t estep = a.out_nhwc ? 1 : ohw;
+        for (int tap = 0; tap < kTcMaxTaps; tap++) p_tap[tap] = tap < KHW ? (uint32_t)a.tap_off[tap] : 0u;
+        const uint64_t dp_proto = desc_interleaved(saddr(smem), (uint32_t)a.rows_a * 16);
+        const uint32_t dp_hi = (uint32_t)(dp_proto >> 32);
+        const uint32_t sf = tmem_base + kTcColSf;
+        auto commit = [&](uint64_t *bar) { // arrives on the barrier when every MMA issued so far has completed
+            asm volatile("{\n\t.reg .pred e;\n\telect.sync _|e, 0xffffffff;\n\t"
+                         "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(saddr(bar))
+                         : "memory");
+        };
+        auto issue_unit = [&](int buf, int u, int ck) {
+            const uint32_t dp_lo = (uint32_t)dp_proto + (uint32_t)buf * (a_bytes >> 4) + (uint32_t)(u * kTcUnit);
+            const uint32_t w_lo = tmem_base + kTcColA + (uint32_t)(buf * kTcMaxWords * kTcWordCols);
+            const uint32_t d_addr = tmem_base + (uint32_t)(u * kTcUnit);
+            const int words = a.CW - ck * KWC; // words left in this chunk; an odd last one is paired with a zero word
+            const uint32_t first_acc = ck > 0 ? 1u : 0u;
 #pragma unroll
-                    for (int j = 0; j < 64; j++) {
-                        const uint32_t v = (acc[j >> 1] >> (16 * (j & 1))) & 0xffffu;
-                        if (co0 + j < a.Co && v != 0u) {
-                            const uintptr_t addr = reinterpret_cast<uintptr_t>(dst + e0 + (size_t)j * estep);
-                            atomicAdd(reinterpret_cast<unsigned int *>(addr & ~(uintptr_t)3), v << ((addr & 2u) * 8u));
-                        }
+            for (int tap = 0; tap < (KHW_T ? KHW_T : kTcMaxTaps); tap++) {
+                if (KHW_T || tap < a.KHW) {
+#pragma unroll
+                    for (int k = 0; k < KWC; k += 2) {
+                        if (k > 0 && k >= words) break;
+                        const uint32_t plo = dp_lo + p_tap[tap] + (uint32_t)k * (uint32_t)a.rows_a;
+                        const uint32_t wcol = w_lo + (uint32_t)((tap * KWC + k) * kTcWordCols);
+                        const uint32_t accumulate = (tap > 0 || k > 0) ? 1u : first_acc;
+                        asm volatile(
+                            "{\n\t.reg .pred p, e;\n\t.reg .b64 db;\n\t"
+                            "mov.b64 db, {%2, %3};\n\t"
+                            "setp.ne.b32 p, %5, 0;\n\t"
+                            "elect.sync _|e, 0xffffffff;\n\t"
+                            "@e tcgen05.mma.cta_group::1.kind::mxf4.block_scale.scale_vec::2X [%0], [%1], db, %4, [%6], [%6], p;\n\t}"
+                            ::"r"(d_addr), "r"(wcol), "r"(plo), "r"(dp_hi), "r"(idesc), "r"(accumulate), "r"(sf)
+                            : "memory");
                     }
-                } else if (a.out_nhwc) {
-                    int16_t *row = dst + m * a.Co + co0;
-                    if (shared_tile) {
-                        // partial sums of this share of the slots: two int16 per 32-bit add, no carry can cross the
-                        // halves because the complete sums fit 16 bits (the host cuts tiles for aligned rows only)
-                        unsigned int *row32 = reinterpret_cast<unsigned int *>(row);
-#pragma unroll
-                        for (int j = 0; j < 32; j++) atomicAdd(row32 + j, acc[j]);
-                    } else if (a.out_vec && (a.Co & 7) == 0 && co0 + kTcCout <= a.Co) {
-#pragma unroll
-                        for (int j = 0; j < 32; j += 4)
-                            *reinterpret_cast<uint4 *>(row + 2 * j) = make_uint4(acc[j], acc[j + 1], acc[j + 2], acc[j + 3]);
-                    } else {
-#pragma unroll
-                        for (int j = 0; j < 64; j++)
-                            if (co0 + j < a.Co) row[j] = (int16_t)((acc[j >> 1] >> (16 * (j & 1))) & 0xffffu);
-                    }
-                } else {
-#pragma unroll
-                    for (int j = 0; j < 64; j++)
-                        if (co0 + j < a.Co)
-                            dst[((size_t)n * a.Co + co0 + j) * ohw + (size_t)oh * a.OW + ow] =
-                                (int16_t)((acc[j >> 1] >> (16 * (j & 1))) & 0xffffu);
                 }
             }
-        }
-#pragma unroll
-        for (int j = 0; j < 32; j++) acc[j] = 0u;
-    };
-    if (warp >= kTcWorkers / 32) {
-        // ---- MMA-issuing warps: operands ready -> accumulator free -> issue -> commit ----
+        };
         int s = 0, ck = 0; // slot (counted through all tiles) and chunk of the step
         for (int step = 0; step < total_steps; step++) {
             if (!wait_on(&bar_full[step & 1], step >> 1)) { failed = true; break; }
-            if (ck == 0 && s >= 2 && !wait_on(&bar_tfree[s & 1], (s >> 1) - 1)) { failed = true; break; }
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            issue_mmas(step, s, ck);
+#pragma unroll
+            for (int u = 0; u < 2; u++) {
+                if (ck == 0 && s > 0 && !wait_on(&bar_tfree[u], s - 1)) { failed = true; break; }
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                issue_unit(step & 1, u, ck);
+                if (ck == a.CK - 1) commit(&bar_done[u]);
+            }
+            if (failed) break;
+            commit(&bar_empty[step & 1]);
             if (++ck == a.CK) { ck = 0; s++; }
         }
         // Whatever way the loop ended: arrive on the drain barrier once all MMAs this warp has issued are complete,
         // so that tensor memory is not released under an MMA still in flight after a timed-out wait.
-        asm volatile("{\n\t.reg .pred e;\n\telect.sync _|e, 0xffffffff;\n\t"
-                     "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(saddr(bar_drain))
-                     : "memory");
-    } else {
-        // ---- expanding / folding warps ----
-        load_tile(0);
-        load_bits();
-        expand_bits(0);
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        warp_arrive(&bar_full[0]);
-        if (total_steps > 1) load_bits();
-        int s_prev = 0, ck_prev = -1; // slot (counted through all tiles) and chunk of step - 1
-        int tile_prev = 0, slots_left_prev = slot_hi(0) - slot_lo(0); // tile of step - 1, its slots still to fold
-        for (int step = 0; step <= total_steps; step++) {
-            // the previous step's MMAs: its operand buffer is free again and, after the last chunk of a slot, the
-            // slot's counts are complete
-            if (step > 0) {
-                if (!wait_on(&bar_empty[(step - 1) & 1], (step - 1) >> 1)) { failed = true; break; }
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            }
-            if (step + 1 < total_steps) {
-                expand_bits((step + 1) & 1);
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                warp_arrive(&bar_full[(step + 1) & 1]);
-                if (step + 2 < total_steps) load_bits();
-            }
-            // fold the slot that the previous step completed and hand its accumulators back
-            if (ck_prev == a.CK - 1) {
-                slot_epilogue(s_prev & 1);
-                warp_arrive(&bar_tfree[s_prev & 1]);
-                if (--slots_left_prev == 0) {
-                    store_tile(tile_prev);
-                    tile_prev++;
-                    slots_left_prev = slot_hi(tile_prev) - slot_lo(tile_prev);
+        commit(bar_drain);
+    } else if (warp == kTcLoadWarp) {
+        // ---- loading warp: weight bit words -> ring, up to a.depth steps ahead ----
+        const int my_tiles = run.tiles;
+        int d = 0, round = 0, issued = 0;
+        for (int k = 0; k < my_tiles && !failed; k++) {
+            long long o0;
+            int nc;
+            tile_origin(k, o0, nc);
+            for (int slot = slot_lo(k); slot < slot_hi(k) && !failed; slot++) {
+                const uint32_t *src = Wb + ((size_t)nc * a.slots + slot) * kTcN * (size_t)(KHW * a.CW);
+                for (int ck = 0; ck < a.CK; ck++, issued++) {
+                    if (round > 0 && !wait_on(&bar_wfree[d], round - 1)) { failed = true; break; }
+                    if (lane == 0) {
+                        const int words = a.CW - ck * KWC < KWC ? a.CW - ck * KWC : KWC; // of the chunk
+                        const uint32_t bytes = (uint32_t)words * kTcN * 4, bar = saddr(&bar_wfull[d]);
+                        const uint32_t dst = saddr(w_ring + d * (KHW * KWC * kTcN));
+                        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes * (uint32_t)KHW) : "memory");
+                        auto copy = [&](uint32_t to, const uint32_t *from, uint32_t n) {
+                            asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                                         ::"r"(to), "l"(from), "r"(n), "r"(bar) : "memory");
+                        };
+                        if (a.CW == KWC) copy(dst, src, bytes * (uint32_t)KHW); // the slot's words are one run
+                        else
+                            for (int tap = 0; tap < KHW; tap++)
+                                copy(dst + (uint32_t)(tap * KWC * kTcN * 4), src + ((size_t)tap * a.CW + ck * KWC) * kTcN, bytes);
+                    }
+                    __syncwarp();
+                    ring_next(d, round);
                 }
             }
-            if (++ck_prev == a.CK) { ck_prev = 0; s_prev++; }
+        }
+        // no copy may still be on its way when the CTA exits (after a time-out; otherwise all have been consumed)
+        for (int j = issued > a.depth ? issued - a.depth : 0; j < issued; j++)
+            if (!wait_on(&bar_wfull[j % a.depth], j / a.depth)) failed = true;
+    } else if (warp >= kTcIssueWarp) {
+        // (idle)
+    } else if (warp >= kTcFoldWarps) {
+        // ---- expanding warps: bit words -> operands ----
+        // Two warps per TMEM lane quarter: they share a weight row's words (even ones, odd ones) and the patch rows.
+        //   weights: row = this thread's TMEM lane, words read from the loading warp's ring
+        //   patch:   row g = et + 256 * r of the residue planes; every thread copies its own rows' words into its own
+        //            places of the ring, a.depth - 1 steps ahead, with asynchronous 4-byte copies (zeros where there is
+        //            no pixel or no channel).  The copies walk the steps in order, the step-dependent part of every
+        //            address is a running pointer.
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kTcRegsExpand));
+        constexpr int kTaps = KHW_T ? KHW_T : kTcMaxTaps, kRows = kTcExpandWarps * 32;
+        const int et = tid - kTcFoldWarps * 32, w_row = et & (kTcN - 1), w_par = (warp >> 2) & 1;
+        const int my_tiles = run.tiles;
+        const uint32_t *a_plane = Ab;
+        uint32_t a_off[RA]; // stored-grid position of the thread's patch rows, ~0u: outside the tensor
+        int ld_ck = 0, ld_left = 0, ld_tile = -1, ld_d = 0, ld_round = 0;
+        // point the loads at the first slot and chunk of tile k of this CTA
+        auto load_tile = [&](int k) {
+            long long o0;
+            int nc;
+            tile_origin(k, o0, nc);
+            const int slot0 = slot_lo(k);
+            ld_tile = k;
+            ld_ck = 0;
+            ld_left = (slot_hi(k) - slot0) * a.CK;
+            a_plane = Ab + (size_t)slot0 * a.CW * a.NHWp;                   // bit plane of the first slot, word 0
+#pragma unroll
+            for (int r = 0; r < RA; r++) {
+                const int g = et + kRows * r;
+                a_off[r] = ~0u;
+                if (g < a.rows_a) {
+                    const int plane = g / a.Mh, q = g - plane * a.Mh;
+                    // candidate indices fit 31 bits (checked on the host); rows before the first stored pixel wrap
+                    // around to large values and are zero like the rows behind the last one
+                    const uint32_t o = (uint32_t)o0 + (uint32_t)q - (uint32_t)a.shift;
+                    if (o < (uint32_t)a.total_o) {
+                        const uint32_t t = o / (uint32_t)a.Wo, j = o - t * (uint32_t)a.Wo;
+                        const uint32_t n = t / (uint32_t)a.Ho, i = t - n * (uint32_t)a.Ho;
+                        const int rh = plane / a.nrw, rw = plane - rh * a.nrw;
+                        a_off[r] = (n * (uint32_t)a.Hrows + i * (uint32_t)a.nrh + (uint32_t)rh) * (uint32_t)a.Wrow +
+                                   (uint32_t)(rw * a.Wq) + j; // < NHWp < 2^32
+                    }
+                }
+            }
+        };
+        // start the copies of the next step (none behind the last one: the group is then empty)
+        auto load_bits = [&]() {
+            if (ld_left > 0) {
+                const int words_left = a.CW - ld_ck * KWC; // words of this chunk that exist; the others are zero
+                const uint32_t dst0 = saddr(p_ring + ld_d * (RA * KWC * kRows) + et);
+#pragma unroll
+                for (int r = 0; r < RA; r++)
+#pragma unroll
+                    for (int k = 0; k < KWC; k++) {
+                        const bool ok = a_off[r] != ~0u && k < words_left;
+                        asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst0 + (uint32_t)((r * KWC + k) * kRows * 4)),
+                                     "l"(ok ? a_plane + (size_t)k * a.NHWp + a_off[r] : Ab), "r"(ok ? 4 : 0) : "memory");
+                    }
+                // advance: next chunk of the slot, or chunk 0 of the next slot
+                if (++ld_ck == a.CK) {
+                    ld_ck = 0;
+                    a_plane += (size_t)(a.CW - KWC * (a.CK - 1)) * a.NHWp;
+                } else {
+                    a_plane += (size_t)KWC * a.NHWp;
+                }
+                if (--ld_left == 0 && ld_tile + 1 < my_tiles) load_tile(ld_tile + 1); // the next call fetches the next tile
+                ring_next(ld_d, ld_round);
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        };
+        const uint32_t w_dst0 = tmem_base + kTcColA + lane_quarter + (uint32_t)(w_par * kTcWordCols);
+        const uint32_t a_kcol = (uint32_t)a.rows_a * 16;
+        auto expand_bits = [&](int buf, int d, int words) { // words: of this chunk; an odd last one gets a zero partner
+            const uint32_t w_dst = w_dst0 + (uint32_t)(buf * kTcMaxWords * kTcWordCols);
+            const uint32_t *w_src = w_ring + d * (KHW * KWC * kTcN) + w_par * kTcN + w_row;
+            const uint32_t *p_src = p_ring + d * (RA * KWC * kRows) + et;
+            uint8_t *a_s = smem + (uint32_t)buf * a_bytes + (uint32_t)et * 16;
+#pragma unroll
+            for (int tap = 0; tap < kTaps; tap++) {
+                if (KHW_T || tap < KHW) {
+#pragma unroll
+                    for (int k = 0; k < KWC; k += 2) {
+                        const uint4 v = spread_weights(k + w_par < words ? w_src[(tap * KWC + k) * kTcN] : 0u);
+                        asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1, %2, %3, %4};"
+                                     ::"r"(w_dst + (uint32_t)((tap * KWC + k) * kTcWordCols)), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+                    }
+                }
+            }
+#pragma unroll
+            for (int r = 0; r < RA; r++) {
+                if (et + kRows * r < a.rows_a) {
+                    uint8_t *dst = a_s + r * (kRows * 16);
+#pragma unroll
+                    for (int k = 0; k < KWC; k++)
+                        *reinterpret_cast<uint4 *>(dst + k * a_kcol) = spread_pixels(p_src[(r * KWC + k) * kRows]);
+                }
+            }
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        };
+        load_tile(0);
+        for (int i = 0; i < a.depth - 1; i++) load_bits();
+        int ck = 0, d = 0, round = 0;
+        for (int step = 0; step < total_steps; step++) {
+            load_bits(); // a.depth - 1 steps ahead; its ring entry is the one this thread emptied in the step before
+            if (a.depth == kTcMaxDepth) asm volatile("cp.async.wait_group %0;" ::"n"(kTcMaxDepth - 1) : "memory");
+            else asm volatile("cp.async.wait_group 1;" ::: "memory");
+            if (!wait_on(&bar_wfull[d], round)) { failed = true; break; }
+            if (step >= 2) { // the MMAs that read this buffer two steps ago
+                if (!wait_on(&bar_empty[step & 1], (step >> 1) - 1)) { failed = true; break; }
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            }
+            expand_bits(step & 1, d, a.CW - ck * KWC);
+            warp_arrive(&bar_full[step & 1]);
+            if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(saddr(&bar_wfree[d])) : "memory");
+            ring_next(d, round);
+            if (++ck == a.CK) ck = 0;
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+    } else {
+        // ---- folding warps: counts -> min(count, n) -> running sums -> outputs ----
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kTcRegsFold));
+        // Warps 0-7 fold unit 0 while the tensor core is on unit 1, warps 8-15 the other way round.  This thread owns one
+        // weight row (lane 32*(warp%4)+lane = sign and output channel) and kTcCols candidates of its unit; two running
+        // sums per register: fp16 (exact up to 2048) or, where they can be larger, 16-bit integers.
+        uint32_t sum[kTcCols / 2];
+#pragma unroll
+        for (int j = 0; j < kTcCols / 2; j++) sum[j] = 0u;
+        const int u = warp >> 3, col0 = ((warp >> 2) & 1) * kTcCols; // unit, first column of the warp in it
+        const uint32_t taddr = tmem_base + lane_quarter + (uint32_t)(u * kTcUnit + col0);
+        // fp16: the conversion rounds counts above 2048, which keeps them above every n it is used with; conversion,
+        // minimum and addition take one instruction per two counts.
+        const __half2 n2h = __half2half2(__int2half_rn(a.wide ? 0 : a.n_or));
+        const uint32_t n2i = (uint32_t)a.n_or * 0x00010001u;
+        auto add16 = [&](uint32_t *sum8, const uint32_t (&x)[16]) {
+            if (!a.wide) {
+#pragma unroll
+                for (int j = 0; j < 8; j++) {
+                    const __half2 cnt = __floats2half2_rn(__uint_as_float(x[2 * j]), __uint_as_float(x[2 * j + 1]));
+                    __half2 t = *reinterpret_cast<__half2 *>(&sum8[j]);
+                    t = __hadd2(t, __hmin2(cnt, n2h));
+                    sum8[j] = *reinterpret_cast<uint32_t *>(&t);
+                }
+            } else { // + 2^23 puts the integer into the low bits of the float
+#pragma unroll
+                for (int j = 0; j < 8; j++) {
+                    const uint32_t cnt = __byte_perm(__float_as_uint(__uint_as_float(x[2 * j]) + 8388608.0f),
+                                                     __float_as_uint(__uint_as_float(x[2 * j + 1]) + 8388608.0f), 0x5410);
+                    sum8[j] += __vminu2(cnt, n2i);
+                }
+            }
+        };
+        // A TMEM read takes some 250 clk while MMAs run, so few reads are waited for: 48 columns, then 32 whose latency
+        // the arithmetic on the first ones covers.
+        auto fold_slot = [&]() {
+            uint32_t x0[16], x1[16], x2[16];
+            REXSC_TMEM_LD16(x0, taddr);
+            REXSC_TMEM_LD16(x1, taddr + 16u);
+            REXSC_TMEM_LD16(x2, taddr + 32u);
+            REXSC_TMEM_WAIT16(x0);
+            REXSC_TMEM_WAIT16(x1);
+            REXSC_TMEM_WAIT16(x2);
+            add16(sum, x0);
+            REXSC_TMEM_LD16(x0, taddr + 48u);
+            add16(sum + 8, x1);
+            REXSC_TMEM_LD16(x1, taddr + 64u);
+            add16(sum + 16, x2);
+            REXSC_TMEM_WAIT16(x0);
+            REXSC_TMEM_WAIT16(x1);
+            // the last counts are in registers: hand the accumulators back
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            warp_arrive(&bar_tfree[u]);
+            add16(sum + 24, x0);
+            add16(sum + 32, x1);
+        };
+        static_assert(kTcCols == 80, "fold_slot reads 5 x 16 columns");
+        // Running sums -> int16 outputs, after the last slot of tile k.  A warp holds 32 output channels of one sign x
+        // kTcCols candidates; they pass through its staging rows, 32 at a time, so that stores run along channels
+        // (channels_last) or along pixels (channel-planar).  A candidate (i, j) of the origin grid is an output pixel
+        // iff i < OH and j < OW.
+        uint32_t *stage = stage_all + warp * (32 * kTcStagePitch);
+        const uint16_t *stage16 = reinterpret_cast<const uint16_t *>(stage);
+        auto store_tile = [&](int k) {
+            long long o0;
+            int nc;
+            tile_origin(k, o0, nc);
+            const bool shared_tile = slot_hi(k) - slot_lo(k) < a.slots; // other CTAs hold the tile's other time slots
+            const int row0 = (warp & 3) * 32;
+            const int co0 = nc * kTcCout + (row0 & (kTcCout - 1));     // channel of the warp's first row
+            int16_t *dst = row0 >= kTcCout ? out_neg : out_pos;
+            const size_t ohw = (size_t)a.OH * a.OW;
+#pragma unroll
+            for (int h = 0; h < kTcCols; h += kTcStageCols) {
+                constexpr int kS = kTcStageCols;
+                const int cnt = kTcCols - h < kS ? kTcCols - h : kS;
+                __syncwarp();
+#pragma unroll
+                for (int j = 0; j < kS / 2; j++) {
+                    if (h / 2 + j >= kTcCols / 2) break;
+                    uint32_t v = sum[h / 2 + j];
+                    if (!a.wide) {
+                        const __half2 t = *reinterpret_cast<const __half2 *>(&v);
+                        v = (uint32_t)__half2ushort_rn(__low2half(t)) | ((uint32_t)__half2ushort_rn(__high2half(t)) << 16);
+                    }
+                    stage[lane * kTcStagePitch + j] = v;
+                    sum[h / 2 + j] = 0u;
+                }
+                __syncwarp();
+                // lane l decodes candidate h + l: element of channel 0, -1: no output pixel
+                long long base = -1;
+                const uint32_t o = (uint32_t)o0 + (uint32_t)(u * kTcUnit + col0 + h + lane);
+                if (lane < cnt && o < (uint32_t)a.total_o) {
+                    const uint32_t t = o / (uint32_t)a.Wo, n = t / (uint32_t)a.Ho;
+                    const int ow = (int)(o - t * (uint32_t)a.Wo), oh = (int)(t - n * (uint32_t)a.Ho);
+                    if (ow < a.OW && oh < a.OH) {
+                        const size_t pix = (size_t)oh * a.OW + ow;
+                        base = (long long)(a.out_nhwc ? ((size_t)n * ohw + pix) * a.Co : (size_t)n * a.Co * ohw + pix);
+                    }
+                }
+                if (a.balanced != 2 && a.out_nhwc && a.out_al4 && (a.Co & 1) == 0) {
+                    // two channels per lane, two pixels per store
+                    const int w = lane & 15, hp = lane >> 4;
+#pragma unroll 4
+                    for (int p = hp; p < cnt; p += 2) {
+                        const long long b = __shfl_sync(0xffffffffu, base, p);
+                        if (b >= 0 && co0 + 2 * w < a.Co) {
+                            const uint32_t v = (uint32_t)stage16[(2 * w) * (2 * kTcStagePitch) + p] |
+                                               ((uint32_t)stage16[(2 * w + 1) * (2 * kTcStagePitch) + p] << 16);
+                            uint32_t *q = reinterpret_cast<uint32_t *>(dst + b + co0 + 2 * w);
+                            // partial sums of this share of the slots: two int16 per 32-bit add, no carry can cross
+                            // the halves because the complete sums fit 16 bits (the host cuts tiles for aligned rows only)
+                            if (shared_tile) atomicAdd(q, v);
+                            else *q = v;
+                        }
+                    }
+                } else {
+                    // One value per lane.  balanced == 2: EVERY tile of the launch adds its sums into outputs that the
+                    // host cleared, one 16-bit value per 32-bit atomic add on the word that holds it (no carry leaves
+                    // the value's half: the complete sums fit 16 bits; the word's other half gets + 0).  All accesses to
+                    // these words are atomic adds, so neighbours stored by other CTAs cannot be lost.
+                    auto put = [&](long long e, uint32_t v) {
+                        if (a.balanced == 2) {
+                            if (v != 0u) {
+                                const uintptr_t addr = reinterpret_cast<uintptr_t>(dst + e);
+                                atomicAdd(reinterpret_cast<unsigned int *>(addr & ~(uintptr_t)3), v << ((addr & 2u) * 8u));
+                            }
+                        } else {
+                            dst[e] = (int16_t)v;
+                        }
+                    };
+                    if (a.out_nhwc) {
+#pragma unroll 4
+                        for (int p = 0; p < cnt; p++) { // lane = channel
+                            const long long b = __shfl_sync(0xffffffffu, base, p);
+                            if (b >= 0 && co0 + lane < a.Co) put(b + co0 + lane, stage16[lane * (2 * kTcStagePitch) + p]);
+                        }
+                    } else { // lane = candidate; half a group of candidates leaves room for two channels
+                        const int rows = 32 / cnt, p = lane % cnt;
+                        const long long b = __shfl_sync(0xffffffffu, base, p);
+#pragma unroll 4
+                        for (int r = lane / cnt; r < 32; r += rows)
+                            if (b >= 0 && co0 + r < a.Co)
+                                put(b + (long long)((size_t)(co0 + r) * ohw), stage16[r * (2 * kTcStagePitch) + p]);
+                    }
+                }
+            }
+        };
+        int s = 0; // slot, counted through all tiles
+        for (int k = 0; k < run.tiles && !failed; k++) {
+            const int n_slots = slot_hi(k) - slot_lo(k);
+            for (int i = 0; i < n_slots && !failed; i++, s++) {
+                if (!wait_on(&bar_done[u], s)) { failed = true; break; }
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                fold_slot();
+                if (i == n_slots - 1) store_tile(k);
+            }
         }
     }
     if (failed && lane == 0) atomicExch(status, 4);
@@ -590,7 +707,6 @@ sc_conv_tc_kernel(TcArgs a, const uint32_t *__restrict__ Ab, const uint32_t *__r
     }
 }
 
-// Tensor-pipe issue-rate probe: back-to-back int8 MMAs (M128 x N x K32) on fixed shared-memory operands.
 // Zeroes the output rows of every tile that two CTAs of a balanced launch share (see TcArgs::balanced).  Block b looks
 // at the cut between runs b and b + 1; a cut inside a tile makes that tile shared.  `grid` is the conv launch's grid.
 __global__ void __launch_bounds__(kTcM)
@@ -626,6 +742,7 @@ zero_shared_tiles_kernel(TcArgs a, int grid, int16_t *__restrict__ out_pos, int1
     }
 }
 
+// Tensor-pipe issue-rate probe: back-to-back int8 MMAs (M128 x N x K32) on fixed shared-memory operands.
 __global__ void __launch_bounds__(128, 2) mma_probe_kernel(int iters, int n_cols, uint32_t *sink)
 {
     extern __shared__ __align__(16) uint8_t smem_raw[];
@@ -680,7 +797,7 @@ __global__ void __launch_bounds__(128, 2) mma_probe_kernel(int iters, int n_cols
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     uint32_t v[16];
-    REXSC_TMEM_LD16_PACKED(v, tmem_base + ((uint32_t)(warp * 32) << 16));
+    REXSC_TMEM_LD16(v, tmem_base + ((uint32_t)(warp * 32) << 16));
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
     sink[blockIdx.x * blockDim.x + tid] = v[0] + (ok ? 0u : 0x80000000u);
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -692,7 +809,7 @@ __global__ void __launch_bounds__(128, 2) mma_probe_kernel(int iters, int n_cols
 // geometry of the tensor-core kernel for one plan; ok = false when the layer does not fit
 struct TcGeom {
     bool ok;
-    int planes, Ho, Wo, Mh, rows_a, KWc, CK, CW;
+    int planes, Ho, Wo, Mh, rows_a, KWc, CK, CW, ra, depth;
     size_t smem;
     int tap_off[kTcMaxTaps];
 };
@@ -713,7 +830,7 @@ TcGeom tc_geometry(const ConvPlan &p)
         }
     g.Mh = (kTcM + max_shift + 7) / 8 * 8;
     g.rows_a = g.planes * g.Mh;
-    if (g.rows_a > kTcMaxARows * kTcWorkers) return g;
+    if (g.rows_a > kTcMaxARows * (kTcExpandWarps * 32)) return g;
     for (int t = 0; t < kTcMaxTaps; t++) g.tap_off[t] = 0;
     for (int kh = 0; kh < p.KH; kh++)
         for (int kw = 0; kw < p.KW; kw++) {
@@ -721,17 +838,22 @@ TcGeom tc_geometry(const ConvPlan &p)
             g.tap_off[kh * p.KW + kw] = plane * g.Mh + (kh / p.sh) * g.Wo + kw / p.sw;
         }
     g.CW = (p.C + 31) / 32;
-    for (int kwc = g.CW >= 2 ? 2 : 1; kwc >= 1; kwc--) {
-        const size_t need = 2 * ((size_t)2 * kwc * g.rows_a * 16 + (size_t)p.KHW * 2 * kwc * kTcN * 16) + 8 * 8 + 8 + sizeof(TileRun) + 128;
-        if (need <= 227 * 1024 && p.KHW * kwc <= 4 * kTcMaxBWords) {
-            g.KWc = kwc;
-            g.CK = (g.CW + kwc - 1) / kwc;
-            // the kernel owns the SM's whole tensor memory: ask for enough shared memory that no second CTA is co-scheduled
-            g.smem = need > 120 * 1024 ? need : 120 * 1024;
-            g.ok = true;
-            break;
-        }
-    }
+    // Words per pipeline step: two (one MMA per tap and unit), and for 1x1 filters, whose steps are short, as many as
+    // the layer has up to eight.
+    g.KWc = p.KHW == 1 ? (g.CW <= 2 ? 2 : g.CW <= 4 ? 4 : 8) : 2;
+    if (p.KHW * g.KWc > kTcMaxWords) return g;
+    g.CK = (g.CW + g.KWc - 1) / g.KWc;
+    g.ra = (g.rows_a + kTcExpandWarps * 32 - 1) / (kTcExpandWarps * 32);
+    g.ra = p.KHW == 1 || g.ra <= 2 ? 2 : g.ra <= 6 ? 6 : kTcMaxARows; // the instantiated row counts
+    auto need = [&](int depth) {
+        return 2 * (size_t)g.KWc * g.rows_a * 16 + (size_t)kTcFoldWarps * 32 * kTcStagePitch * 4 +
+               (size_t)depth * g.KWc * 4 * (p.KHW * kTcN + g.ra * kTcExpandWarps * 32) + kTcBars * 8 + 8 + sizeof(TileRun) + 128;
+    };
+    g.depth = need(kTcMaxDepth) <= 227 * 1024 ? kTcMaxDepth : 2;
+    if (need(g.depth) > 227 * 1024) return g;
+    // the kernel owns the SM's whole tensor memory: ask for enough shared memory that no second CTA is co-scheduled
+    g.smem = need(g.depth) > 120 * 1024 ? need(g.depth) : 120 * 1024;
+    g.ok = true;
     return g;
 }
 
@@ -754,7 +876,7 @@ bool conv_tc_supported(const ConvPlan &p)
     if (!g.ok) return false;
     const long long cap = p.n_or < p.Kdot ? p.n_or : p.Kdot;                   // largest per-slot contribution
     if ((long long)p.words * 32 * cap > 65535) return false;                  // 16-bit running sums
-    if (((long long)p.Kdot << kTcScaleLog2) > 65535) return false;            // 16-bit packed accumulator reads
+    if (p.Kdot > 8191) return false;                                          // (far below what fp32 counts exactly)
     if (p.Kdot > (1 << 24)) return false;
     const long long total_o = (long long)p.N * g.Ho * g.Wo;
     if (total_o + kTcM > 0x7fffffffLL) return false;                          // 31-bit candidate indices
@@ -797,7 +919,7 @@ int launch_conv_tc(const ConvPlan &p, const rexsc_sc_conv_desc &d, void *d_tc_ws
     const uint32_t *Wb = reinterpret_cast<const uint32_t *>(static_cast<const uint8_t *>(d_tc_ws) + weight_offset);
     TcArgs a;
     a.OH = p.OH; a.OW = p.OW; a.KHW = p.KHW; a.Co = p.Co;
-    a.CW = CW; a.KWc = g.KWc; a.CK = g.CK;
+    a.CW = CW; a.KWc = g.KWc; a.CK = g.CK; a.depth = g.depth;
     a.nrh = p.nrh; a.nrw = p.nrw; a.Wq = p.Wq; a.Hrows = p.Hrows; a.Wrow = p.Wrow;
     a.Ho = g.Ho; a.Wo = g.Wo; a.Mh = g.Mh; a.rows_a = g.rows_a;
     a.shift = p.origin ? g.Wo + 1 : 0;
@@ -822,8 +944,8 @@ int launch_conv_tc(const ConvPlan &p, const rexsc_sc_conv_desc &d, void *d_tc_ws
     // time goes to the per-slot hand-offs, and the atomic stores of the cut tiles cost more than the idle SMs did)
     const bool heavy_slots = p.KHW * CW >= 16 || a.total_tiles < sms;
     if (allow_balanced && heavy_slots && rows_ok && gate >= 0 && a.total_tiles % sms != 0) {
-        // short layers: as many CTAs as leaves each about 64 pipeline steps to amortise its prologue
-        long long ctas = units * g.CK / 64;
+        // short layers: as many CTAs as leaves each about four slots to amortise its prologue
+        long long ctas = units / 4;
         if (ctas < 1) ctas = 1;
         if (ctas > sms) ctas = sms;
         const long long waves = (a.total_tiles + sms - 1) / sms;
@@ -839,7 +961,7 @@ int launch_conv_tc(const ConvPlan &p, const rexsc_sc_conv_desc &d, void *d_tc_ws
     const size_t out_elems = (size_t)p.M * p.Co;
     if (allow_balanced && heavy_slots && !rows_ok && aligned4 && (out_elems & 1) == 0 && out_elems * sizeof(int16_t) <= ((size_t)16 << 20) &&
         gate >= 0 && a.total_tiles % sms != 0) {
-        long long ctas = units * g.CK / 64;
+        long long ctas = units / 4;
         if (ctas < 1) ctas = 1;
         if (ctas > sms) ctas = sms;
         const long long waves = (a.total_tiles + sms - 1) / sms;
@@ -856,21 +978,17 @@ int launch_conv_tc(const ConvPlan &p, const rexsc_sc_conv_desc &d, void *d_tc_ws
     }
     a.NHWp = p.NHWp; a.out_nhwc = d.out_channels_last;
     if ((reinterpret_cast<uintptr_t>(d_pos) | reinterpret_cast<uintptr_t>(d_neg)) & 1u) return REXSC_E_BAD_ARG;
-    a.out_vec = ((reinterpret_cast<uintptr_t>(d_pos) | reinterpret_cast<uintptr_t>(d_neg)) & 15u) == 0 ? 1 : 0;
+    a.out_al4 = aligned4 ? 1 : 0;
     {
         const long long cap = p.n_or < p.Kdot ? p.n_or : p.Kdot;
-        a.descale_each = (((long long)slots * cap) << kTcScaleLog2) > 65535 ? 1 : 0;
+        a.wide = (long long)slots * cap > 2048 ? 1 : 0; // fp16 counts exactly up to 2048
         a.n_or = (int)cap; // a count never exceeds the dot length, so clamping there changes nothing
     }
     for (int t = 0; t < kTcMaxTaps; t++) a.tap_off[t] = g.tap_off[t];
-    const int ra = (g.rows_a + kTcWorkers - 1) / kTcWorkers;
-    auto pick = [&](auto khw_tag) {
-        constexpr int KHW_T = decltype(khw_tag)::value;
-        if (g.KWc == 2) return ra == 1 ? sc_conv_tc_kernel<KHW_T, 2, 1> : sc_conv_tc_kernel<KHW_T, 2, kTcMaxARows>;
-        return ra == 1 ? sc_conv_tc_kernel<KHW_T, 1, 1> : sc_conv_tc_kernel<KHW_T, 1, kTcMaxARows>;
-    };
-    auto kernel = p.KHW == 9 ? pick(std::integral_constant<int, 9>{})
-                : p.KHW == 1 ? pick(std::integral_constant<int, 1>{}) : pick(std::integral_constant<int, 0>{});
+    auto kernel = p.KHW == 9 ? (g.ra == 2 ? sc_conv_tc_kernel<9, 2, 2> : g.ra == 6 ? sc_conv_tc_kernel<9, 2, 6> : sc_conv_tc_kernel<9, 2, kTcMaxARows>)
+                : p.KHW != 1 ? (g.ra == 2 ? sc_conv_tc_kernel<0, 2, 2> : g.ra == 6 ? sc_conv_tc_kernel<0, 2, 6> : sc_conv_tc_kernel<0, 2, kTcMaxARows>)
+                : g.KWc == 2 ? sc_conv_tc_kernel<1, 2, 2>
+                : g.KWc == 4 ? sc_conv_tc_kernel<1, 4, 2> : sc_conv_tc_kernel<1, 8, 2>; // (one plane of kTcM rows)
     REXSC_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g.smem));
     kernel<<<grid, kTcThreads, g.smem, st>>>(a, Ab, Wb, d_pos, d_neg, d_status, gate);
     REXSC_LAUNCH_CHECK("sc_conv_tc_kernel");
