@@ -17,9 +17,9 @@
 namespace rexsc {
 
 // ---- LFSR step: torch_c/sc-extension/sc_device.cuh:108-248 ----------------------------------
-__host__ __device__ __forceinline__ int lfsr_next(int v, int l, int xnor)
+__host__ __device__ constexpr int lfsr_next(int v, int l, int xnor)
 {
-    int fb;
+    int fb = 0;
     switch (l) {
     case 1: return 1 - v;
     case 2: return (v + 1) & 3;
@@ -34,7 +34,47 @@ __host__ __device__ __forceinline__ int lfsr_next(int v, int l, int xnor)
     return ((v << 1) & ((1 << l) - 1)) | fb;
 }
 
-// One thread per (phase, value): run the generator for bit_length steps.
+// The generator's states in the order it visits them, per register length and feedback, worked out by the compiler: the
+// state t steps after a seed is a lookup, so the tables below are filled by as many threads as they have entries instead
+// of by threads that each walk the register.
+struct Orbit {
+    uint8_t state[256]; // state[0] is the start state (XNOR: 0, XOR: 1)
+    uint8_t pos[256];   // position of a state in it
+    int len;
+};
+constexpr Orbit make_orbit(int l, int xnor)
+{
+    Orbit o{};
+    const int start = 1 - xnor;
+    int st = start;
+    do {
+        o.state[o.len] = (uint8_t)st;
+        o.pos[st] = (uint8_t)o.len;
+        o.len++;
+        st = lfsr_next(st, l, xnor);
+    } while (st != start);
+    return o;
+}
+struct Orbits { Orbit o[2][8]; };
+constexpr Orbits make_orbits()
+{
+    Orbits r{};
+    for (int x = 0; x < 2; x++)
+        for (int l = 1; l <= 8; l++) r.o[x][l - 1] = make_orbit(l, x);
+    return r;
+}
+constexpr Orbits kOrbits = make_orbits();
+constexpr bool orbits_cover_all_seeds() // maximal length from 3 bits on; all states at 1 and 2 bits
+{
+    for (int x = 0; x < 2; x++)
+        for (int l = 1; l <= 8; l++)
+            if (kOrbits.o[x][l - 1].len != (l <= 2 ? 1 << l : (1 << l) - 1)) return false;
+    return true;
+}
+static_assert(orbits_cover_all_seeds(), "a seed may lie outside the tabulated cycle");
+__device__ const Orbits d_orbits = make_orbits();
+
+// Table of stream words of every (seed phase, value).
 // Generation loop semantics: torch_c/sc-extension/sc_cuda_conv.cu:70-92 (weights), :149-163 (activations):
 // advance then compare; progressive-loading mask on the value; int8 storage of state and value; for
 // gen_config g the weight bit t lands in slots t*g..t*g+g-1 and the activation bit t in slots
@@ -43,43 +83,48 @@ struct LutParams {
     int l, bit_length, g, xnor, tw, lw, lwait, words;
 };
 
-// stream words of one (seed phase, value) pair into out[0 .. words)
-template <typename Store>
-__device__ __forceinline__ void lut_entry(const LutParams &lp, int is_weight, int phase, int value, Store store)
+// One block per seed phase.  Its threads first note state and value mask of every time slot, then each fills the words
+// of its values.  blockIdx.y = 0: the table `lut` for generator kind `is_weight`; blockIdx.y = 1 (pair launch): the weight
+// table lut_w.  (One thread per entry that ran the generator: 14 us at 32 slots, 53 us for the two 260 KB tables of 128.)
+constexpr int kLutThreads = 128;
+__global__ void __launch_bounds__(kLutThreads) build_lut_kernel(LutParams lp, int is_weight, uint32_t *__restrict__ lut,
+                                                                uint32_t *__restrict__ lut_w)
 {
-    int state = (int)(int8_t)(phase + 1 - (lp.xnor ? 1 : 0));
-    const int val8 = (int)(int8_t)value;
-    uint32_t acc[32]; // words <= 32 (slots <= 1024)
-#pragma unroll 1
-    for (int j = 0; j < lp.words; j++) acc[j] = 0u;
-#pragma unroll 1
-    for (int t = 0; t < lp.bit_length; t++) {
-        int cur = (t / lp.lwait + 1) * lp.lw - 1;
-        if (cur > lp.tw) cur = lp.tw;
-        const int sh = lp.tw - cur;
-        const int actual = (val8 >> sh) << sh;
-        state = (int)(int8_t)lfsr_next(state, lp.l, lp.xnor);
-        if (actual > state) {
-            for (int j = 0; j < lp.g; j++) {
-                const int slot = is_weight ? t * lp.g + j : (t / lp.g) * lp.g * lp.g + j * lp.g + t % lp.g;
-                acc[slot >> 5] |= 1u << (slot & 31);
+    __shared__ int slot_s[1024]; // low half: state (signed), high half: bits of the value masked off
+    if (blockIdx.y == 1) { is_weight = 1; lut = lut_w; }
+    const int nvals = 1 << lp.l, phase = blockIdx.x, g = lp.g;
+    const Orbit &orbit = d_orbits.o[lp.xnor ? 1 : 0][lp.l - 1];
+    const int first = orbit.pos[(phase + 1 - (lp.xnor ? 1 : 0)) & 255] + 1, len = orbit.len;
+    for (int s = threadIdx.x; s < lp.words * 32; s += blockDim.x) {
+        int t = s / g; // the step whose bit lands in slot s
+        bool ok = s < lp.bit_length * g;
+        if (!is_weight) {
+            const int block = s / (g * g);
+            t = block * g + s % g;
+            ok = t < lp.bit_length;
+        }
+        int entry = 127; // no value is above it
+        if (ok) {
+            int cur = (t / lp.lwait + 1) * lp.lw - 1;
+            if (cur > lp.tw) cur = lp.tw;
+            const int sh = lp.tw - cur < 31 ? lp.tw - cur : 31;
+            entry = ((int)(int8_t)orbit.state[(first + t) % len] & 0xffff) | (sh << 16);
+        }
+        slot_s[s] = entry;
+    }
+    __syncthreads();
+    for (int v = threadIdx.x; v < nvals; v += blockDim.x) {
+        const int val8 = (int)(int8_t)v;
+        for (int j = 0; j < lp.words; j++) {
+            uint32_t word = 0u;
+#pragma unroll 8
+            for (int b = 0; b < 32; b++) {
+                const int e = slot_s[j * 32 + b], sh = e >> 16;
+                word |= ((val8 >> sh) << sh) > (int)(int16_t)e ? 1u << b : 0u;
             }
+            lut[((size_t)phase * nvals + v) * lp.words + j] = word;
         }
     }
-    for (int j = 0; j < lp.words; j++) store(j, acc[j]);
-}
-
-// blockIdx.y = 0: the table `lut` for generator kind `is_weight`; blockIdx.y = 1 (pair launch): the weight table lut_w
-__global__ void build_lut_kernel(LutParams lp, int is_weight, uint32_t *__restrict__ lut, uint32_t *__restrict__ lut_w)
-{
-    if (blockIdx.y == 1) { is_weight = 1; lut = lut_w; }
-    const int nvals = 1 << lp.l;
-    const int period = nvals - 1;
-    const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= period * nvals) return;
-    const int phase = idx / nvals;
-    const int value = idx - phase * nvals;
-    lut_entry(lp, is_weight, phase, value, [&](int j, uint32_t v) { lut[(size_t)idx * lp.words + j] = v; });
 }
 
 int launch_build_lut(int l, int bit_length, int gen_config, int xnor, int tw, int lw, int lwait, int is_weight,
@@ -89,9 +134,8 @@ int launch_build_lut(int l, int bit_length, int gen_config, int xnor, int tw, in
     int slots = bit_length * gen_config;
     if (slots > 1024) return REXSC_E_TOO_LONG;
     int words = (slots + 31) / 32;
-    int total = ((1 << l) - 1) * (1 << l);
     LutParams lp{l, bit_length, gen_config, xnor, tw, lw, lwait, words};
-    build_lut_kernel<<<(total + 127) / 128, 128, 0, st>>>(lp, is_weight, d_lut, nullptr);
+    build_lut_kernel<<<(1 << l) - 1, kLutThreads, 0, st>>>(lp, is_weight, d_lut, nullptr);
     REXSC_LAUNCH_CHECK("build_lut_kernel");
     return REXSC_OK;
 }
@@ -104,9 +148,8 @@ int launch_build_lut_pair(int l, int bit_length, int gen_config, int xnor, int t
     const int slots = bit_length * gen_config;
     if (slots > 1024) return REXSC_E_TOO_LONG;
     const int words = (slots + 31) / 32;
-    const int total = ((1 << l) - 1) * (1 << l);
     LutParams lp{l, bit_length, gen_config, xnor, tw, lw, lwait, words};
-    build_lut_kernel<<<dim3((total + 127) / 128, 2), 128, 0, st>>>(lp, 0, d_lut_a, d_lut_w);
+    build_lut_kernel<<<dim3((1 << l) - 1, 2), kLutThreads, 0, st>>>(lp, 0, d_lut_a, d_lut_w);
     REXSC_LAUNCH_CHECK("build_lut_kernel");
     return REXSC_OK;
 }
@@ -735,7 +778,7 @@ expand_act_bits_fast_kernel(ExpandActArgs a, const T *__restrict__ x, const uint
             }
             __syncwarp();
             // ---- lane = pixel: look the 32 channels' stream words up, transpose, store 32 slot words ----
-#pragma unroll
+#pragma unroll 1
             for (int wd = 0; wd < WORDS; wd++) {
                 uint32_t v[32];
 #pragma unroll
@@ -839,7 +882,7 @@ template <typename T, int WORDS, bool NCHW = false>
 __device__ __forceinline__ void expand_act_async_body(const ExpandActArgs &a, const T *__restrict__ x,
                                                       const uint32_t *lut_s, uint8_t *raw_all, int raw_stride,
                                                       ActAsyncShared &sh, uint32_t *__restrict__ Ab, int CW,
-                                                      long long n_groups)
+                                                      long long n_groups, int cw_parts = 1)
 {
     constexpr int E = 16 / (int)sizeof(T), LPP = 32 / E, PPI = 32 / LPP; // elements per lane, lanes per pixel, pixels per pass
     constexpr int kRowBytes = 32 * (int)sizeof(T), kTileBytes = 32 * kRowBytes;
@@ -919,23 +962,29 @@ __device__ __forceinline__ void expand_act_async_body(const ExpandActArgs &a, co
         cp_async_commit();
     };
 
-    long long grp = (long long)blockIdx.x * kFastWarps + warp;
-    if (grp >= n_groups) return; // warp-uniform; no block-wide barrier follows
-    Pix cur = decode(grp, 0), nxt = cur;
+    // An item is a pixel group and one part of its channel words (all of them unless groups are few): item i = part
+    // i % cw_parts of group i / cw_parts.
+    const int part_words = (CW + cw_parts - 1) / cw_parts;
+    const long long n_items = n_groups * cw_parts;
+    auto part_of = [&](long long i) { return cw_parts == 1 ? 0 : (int)(i % cw_parts) * part_words; };
+    long long grp = (long long)blockIdx.x * kFastWarps + warp; // item
+    if (grp >= n_items) return; // warp-uniform; no block-wide barrier follows
+    Pix cur = decode(grp / cw_parts, 0), nxt = cur;
     __syncwarp();
-    issue(0, 0, 0);
+    issue(0, part_of(grp), 0);
     land(0);
     int buf = 0, stage = 0;
     for (;;) {
         const long long grp_next = grp + stride;
-        const bool has_next = grp_next < n_groups;
-        if (has_next) nxt = decode(grp_next, buf ^ 1);
+        const bool has_next = grp_next < n_items;
+        if (has_next) nxt = decode(grp_next / cw_parts, buf ^ 1);
         __syncwarp();
-        for (int cw = 0; cw < CW; cw++) {
+        const int cw_first = part_of(grp), cw_end = cw_first + part_words < CW ? cw_first + part_words : CW;
+        for (int cw = cw_first; cw < cw_end; cw++) {
             // keep the next tile's loads in flight while this one is processed
-            const bool more = cw + 1 < CW || has_next;
-            if (cw + 1 < CW) issue(buf, cw + 1, stage ^ 1);
-            else if (has_next) issue(buf ^ 1, 0, stage ^ 1);
+            const bool more = cw + 1 < cw_end || has_next;
+            if (cw + 1 < cw_end) issue(buf, cw + 1, stage ^ 1);
+            else if (has_next) issue(buf ^ 1, part_of(grp_next), stage ^ 1);
             else if (!kRegStage) cp_async_commit(); // an empty group keeps the wait below uniform
             if (!kRegStage) cp_async_wait_all_but_one();
             __syncwarp();
@@ -964,7 +1013,7 @@ __device__ __forceinline__ void expand_act_async_body(const ExpandActArgs &a, co
             }
             __syncwarp();
             // ---- lane = pixel: look the 32 channels' stream words up, transpose, store 32 slot words ----
-#pragma unroll
+#pragma unroll 1
             for (int wd = 0; wd < WORDS; wd++) {
                 uint32_t v[32];
 #pragma unroll
@@ -1057,42 +1106,54 @@ struct ExpandWBitsArgs {
 // every CTA builds both tables in its own shared memory straight from the LFSR (a few thousand short generator runs
 // per CTA, nothing read from global memory), takes its share of the weight items, then runs the pipelined activation
 // expansion.
-// Table of stream words of every (seed phase, value), built in shared memory without running the generator per entry.
+// Table of stream words of every (seed phase, value), built in shared memory without running the generator.
 // Valid for gen_config 1 with progressive loading inactive (the front end's settings), where the activation and the
-// weight table coincide.  The LFSR visits its states in one cycle c_0, c_1, ...; the generator seeded with state s emits
-// at step t the comparison value > c_{pos(s) + t + 1}, so the word of (phase, value) has bit t set iff that threshold is
-// below the value.  Per phase one thread scatters bit t into the entry `threshold + 1` of its (thread-private) row and
-// then ORs the row's entries cumulatively: entry v ends up holding every bit whose threshold is < v.  Rows are written
-// twice (phase and phase + period) with one word of padding, the layout the expansion kernels index without a modulo.
+// weight table coincide.  The generator seeded with state s emits at step t the comparison value > orbit[pos(s) + t + 1],
+// so the word of (phase, value) has bit t set iff that threshold is below the value: every (phase, step) sets its bit in
+// the entry `threshold + 1` of the phase's row, and an OR scan over the values, one warp per row, completes the entries.
+// Rows are written twice (phase and phase + period) with one word of padding, the layout the expansion kernels index
+// without a modulo.
 template <int WORDS>
 __device__ __forceinline__ void build_doubled_table(const LutParams &lp, int period, int nvals, uint32_t *lut_s,
                                                     uint8_t *cyc_s, uint8_t *pos_s)
 {
-    const int row_words = nvals * WORDS + 1;
-    if (threadIdx.x == 0) {
-        int st = 1 - (lp.xnor ? 1 : 0);
-        for (int k = 0; k < period; k++) {
-            cyc_s[k] = (uint8_t)st;
-            pos_s[st] = (uint8_t)k;
-            st = lfsr_next(st, lp.l, lp.xnor);
-        }
+    const int row_words = nvals * WORDS + 1, lane = threadIdx.x & 31;
+    const Orbit &orbit = d_orbits.o[lp.xnor ? 1 : 0][lp.l - 1];
+    const int len = lp.l <= 2 ? nvals : period; // of the generator's cycle
+    for (int i = threadIdx.x; i < nvals; i += blockDim.x) {
+        cyc_s[i] = orbit.state[i];
+        pos_s[i] = orbit.pos[i];
+    }
+    for (int i = threadIdx.x; i < period * row_words; i += blockDim.x) lut_s[i] = 0u;
+    __syncthreads();
+    for (int i = threadIdx.x; i < period * lp.bit_length; i += blockDim.x) {
+        const int phase = i / lp.bit_length, t = i - phase * lp.bit_length;
+        const int thr = cyc_s[(pos_s[phase + 1 - (lp.xnor ? 1 : 0)] + 1 + t) % len];
+        if (thr + 1 < nvals) atomicOr(&lut_s[phase * row_words + (thr + 1) * WORDS + (t >> 5)], 1u << (t & 31));
     }
     __syncthreads();
-    for (int phase = threadIdx.x; phase < period; phase += blockDim.x) {
+    for (int phase = threadIdx.x >> 5; phase < period; phase += blockDim.x >> 5) {
         uint32_t *row = lut_s + phase * row_words;
-        for (int i = 0; i < nvals * WORDS; i++) row[i] = 0u;
-        int k = pos_s[phase + 1 - (lp.xnor ? 1 : 0)];
-        for (int t = 0; t < lp.bit_length; t++) {
-            if (++k == period) k = 0;
-            const int thr = cyc_s[k];
-            if (thr + 1 < nvals) row[(thr + 1) * WORDS + (t >> 5)] |= 1u << (t & 31);
-        }
-        for (int v = 1; v < nvals; v++)
 #pragma unroll
-            for (int j = 0; j < WORDS; j++) row[v * WORDS + j] |= row[(v - 1) * WORDS + j];
+        for (int j = 0; j < WORDS; j++) {
+            uint32_t below = 0u; // OR of the 32-value groups before
+            for (int v0 = 0; v0 < nvals; v0 += 32) {
+                const int at = (v0 + lane) * WORDS + j;
+                uint32_t x = v0 + lane < nvals ? row[at] : 0u;
+#pragma unroll
+                for (int d = 1; d < 32; d *= 2) {
+                    const uint32_t y = __shfl_up_sync(0xffffffffu, x, d);
+                    if (lane >= d) x |= y;
+                }
+                x |= below;
+                if (v0 + lane < nvals) {
+                    row[at] = x;
+                    if (phase < period - 1) row[period * row_words + at] = x;
+                }
+                below = __shfl_sync(0xffffffffu, x, 31);
+            }
+        }
     }
-    __syncthreads();
-    for (int i = threadIdx.x; i < (period - 1) * row_words; i += blockDim.x) lut_s[period * row_words + i] = lut_s[i];
     __syncthreads();
 }
 
@@ -1106,6 +1167,8 @@ struct ExpandAllArgs {
     int verify_border; // check that the border pixels of the padded activation quantise to zero; status[1] = 1 otherwise
     int gate;          // run only if status[1] != 0
     int verify_vec;    // the border check may use 16-byte loads and 32-bit indices
+    int w_vec;         // fp32 weights, input channels fastest, whole 16-byte groups
+    int cw_parts;      // the channel words of a pixel group are shared out to this many warps
 };
 
 __device__ __forceinline__ float load_weight_any(const void *w, int dtype, long long i)
@@ -1157,35 +1220,30 @@ expand_all_kernel(ExpandAllArgs g, const T *__restrict__ x, const void *__restri
                 }
             }
         } else {
-            const long long total = (long long)a.N * per_img * a.C;
-            for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
-                 idx += (long long)gridDim.x * blockDim.x) {
-                // channel-planar: consecutive threads walk the border pixels of one channel
-                const uint32_t b = (uint32_t)(idx % per_img);
-                const long long t = idx / per_img;
-                const int c = (int)(t % a.C), n = (int)(t / a.C);
+            // one warp per image (channels_last) or image plane (channel-planar); a lane's border pixels are the same in
+            // all of them, so their positions are worked out once
+            const int lane = threadIdx.x & 31;
+            const long long units = NCHW ? (long long)a.N * a.C : (long long)a.N, unit_elems = (long long)a.H * a.W * (NCHW ? 1 : a.C);
+            const long long w0 = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), nw = (long long)gridDim.x * (blockDim.x >> 5);
+            for (uint32_t b = (uint32_t)lane; b < per_img; b += 32) {
                 int hi, wi;
-                if (border_pixel(b, hi, wi)) {
-                    const long long xi = NCHW ? (((long long)n * a.C + c) * a.H + hi) * a.W + wi
-                                              : (((long long)n * a.H + hi) * a.W + wi) * a.C + c;
-                    bad |= load_as_float<T>(x, xi) > 0.f;
-                }
+                if (!border_pixel(b, hi, wi)) continue;
+                const T *px = x + ((long long)hi * a.W + wi) * (NCHW ? 1 : a.C);
+#pragma unroll 4
+                for (long long n = w0; n < units; n += nw)
+                    for (int c = 0; c < (NCHW ? 1 : a.C); c++) bad |= load_as_float<T>(px, n * unit_elems + c) > 0.f;
             }
         }
         if (bad) atomicExch(status + 1, 1);
     }
     build_doubled_table<WORDS>(g.lut, a.period, a.nvals, lut_s, cyc_s, pos_s);
-    // ---- weights: one warp per (block of 32 output channels, tap, channel word); lane = input channel of the word ----
-    // For every output channel of the block the warp looks the 32 channels' stream words up and transposes them across
-    // its lanes (lane = time slot afterwards); the 32 x 32 slot words of the block go through a swizzled tile in the
-    // warp's staging area so that each slot's words leave as one 128-byte run over the output channels.
+    // ---- weights: one warp per (output channel or block of 32 of them, tap, channel word) ----
     {
         const ExpandWBitsArgs &wa = g.w;
         const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
         const int slots = WORDS * 32;
         const size_t row_words_w = (size_t)wa.KHW * wa.CW;
         const int row_words = wa.nvals * WORDS + 1;
-        uint32_t *tile = reinterpret_cast<uint32_t *>(reinterpret_cast<uint8_t *>(lut_s) + lut_smem_bytes) + warp * 2048; // [2][32][32]
         // Small filters: one output channel per item (more items than warps matter more than coalesced stores).  The
         // weight of the warp's NEXT item is loaded before the current one is processed.
         auto fine_weight = [&](long long item) { // lane's weight of a fine item; 0 outside the tensor
@@ -1219,84 +1277,101 @@ expand_all_kernel(ExpandAllArgs g, const T *__restrict__ x, const void *__restri
             const long long seed_ind = wa.linear_seeds ? (long long)ci : ((long long)ci * wa.KH + kh) * wa.KW + kw;
             const int row_off = (int)(((neg ? wa.seed_neg : wa.seed_pos) + seed_ind) % wa.period) * row_words;
             const int nchunk = co >> 6, col = co & 63;
+            const uint32_t signs = reverse_nibbles(__ballot_sync(0xffffffffu, neg));
 #pragma unroll
             for (int wd = 0; wd < WORDS; wd++) {
-                const uint32_t v = lut_s[row_off + mag * WORDS + wd];
+                // a weight has one sign, so the slot words of both signs are one transposed word under the sign mask
+                const uint32_t v = reverse_nibbles(transpose32_warp(lut_s[row_off + mag * WORDS + wd], lane));
                 uint32_t *dst = Wb + (((size_t)nchunk * slots + wd * 32 + lane) * row_words_w + (size_t)tap * wa.CW + cw) * 128 + col;
-                dst[0] = reverse_nibbles(transpose32_warp(neg ? 0u : v, lane));
-                dst[64] = reverse_nibbles(transpose32_warp(neg ? v : 0u, lane));
+                dst[0] = v & ~signs;
+                dst[64] = v & signs;
             }
         }
-        // Large filters: 32 output channels per item, stores coalesced through the tile
+        // Large filters: 32 output channels x 32 input channels of one tap per item, lane = output channel.  A lane looks
+        // the stream words of its 32 input channels up (their seed phases are the same in all lanes), transposes them in
+        // its registers like the activation path, and every slot's words leave as one 128-byte run.  Input channel c goes
+        // to row (c with its low two bits reversed), which leaves the nibbles of the slot words bit-reversed.
         for (long long item = (long long)blockIdx.x * kFastWarps + warp; g.w_coarse && item < g.w_items;
              item += (long long)gridDim.x * kFastWarps) {
             const int cw = (int)(item % wa.CW);
-            long long t = item / wa.CW;
+            const long long t = item / wa.CW;
             const int tap = (int)(t % wa.KHW);
             const int cb = (int)(t / wa.KHW); // block of 32 output channels, 0 .. 2*NC: rows past Co stay zero
             const int kh = tap / wa.KW, kw = tap - kh * wa.KW;
-            const int ci = cw * 32 + lane;
+            const int c0 = cw * 32, co = cb * 32 + lane;
+            const long long w_base = wa.ohwi ? (((long long)co * wa.KH + kh) * wa.KW + kw) * wa.C + c0
+                                             : (((long long)co * wa.C + c0) * wa.KH + kh) * wa.KW + kw;
+            const long long w_step = wa.ohwi ? 1 : wa.KHW;
             // seed index c*KH*KW + kh*KW + kw, offset 13 for both signs (sc_cuda_conv.cu:45,55-56); linear: c only
-            const long long seed_ind = wa.linear_seeds ? (long long)ci : ((long long)ci * wa.KH + kh) * wa.KW + kw;
-            const int row_off_pos = (int)((wa.seed_pos + seed_ind) % wa.period) * row_words;
-            const int row_off_neg = (int)((wa.seed_neg + seed_ind) % wa.period) * row_words;
+            const uint32_t period = (uint32_t)wa.period;
+            const long long seed0 = wa.linear_seeds ? (long long)c0 : ((long long)c0 * wa.KH + kh) * wa.KW + kw;
+            const uint32_t seed_step = (wa.linear_seeds ? 1u : (uint32_t)wa.KHW) % period;
             const int nchunk = cb >> 1, col0 = (cb & 1) * 32;
+            const bool row_ok = co < wa.Co;
+            const bool vec = g.w_vec != 0 && row_ok && c0 + 32 <= wa.C;
 #pragma unroll 1
             for (int wd = 0; wd < WORDS; wd++) {
-                // eight output channels at a time: their loads are issued together, so the item costs four memory
-                // latencies instead of thirty-two
-#pragma unroll 1
-                for (int cl0 = 0; cl0 < 32; cl0 += 8) {
-                    float wv[8];
+                uint32_t v[32], signs = 0u;
+                uint32_t pp = (uint32_t)((wa.seed_pos + seed0) % period), pn = (uint32_t)((wa.seed_neg + seed0) % period);
 #pragma unroll
-                    for (int j = 0; j < 8; j++) {
-                        const int co = cb * 32 + cl0 + j;
-                        wv[j] = 0.f;
-                        if (ci < wa.C && co < wa.Co) {
-                            const long long wi = wa.ohwi ? (((long long)co * wa.KH + kh) * wa.KW + kw) * wa.C + ci
-                                                         : (((long long)co * wa.C + ci) * wa.KH + kh) * wa.KW + kw;
-                            wv[j] = load_weight_any(wt, g.w_dtype, wi);
-                        }
+                for (int b = 0; b < 32; b += 8) { // the loads of eight channels are issued together
+                    float wv[8];
+                    if (vec) {
+                        const float4 *q = reinterpret_cast<const float4 *>(static_cast<const float *>(wt) + w_base + b);
+                        const float4 lo = __ldg(q), hi = __ldg(q + 1);
+                        wv[0] = lo.x; wv[1] = lo.y; wv[2] = lo.z; wv[3] = lo.w;
+                        wv[4] = hi.x; wv[5] = hi.y; wv[6] = hi.z; wv[7] = hi.w;
+                    } else {
+#pragma unroll
+                        for (int k = 0; k < 8; k++)
+                            wv[k] = row_ok && c0 + b + k < wa.C ? load_weight_any(wt, g.w_dtype, w_base + (b + k) * w_step) : 0.f;
                     }
 #pragma unroll
-                    for (int j = 0; j < 8; j++) {
-                        const int cl = cl0 + j;
-                        const float v = wv[j] * wa.scale;
-                        // w_pos = ceil(clamp(v, 0, L-1)); w_neg = ceil(-clamp(v, 1-L, 0))  (sc_cuda.cpp:92-93)
-                        const int qp = (int)ceilf(fminf(fmaxf(v, 0.f), wa.scale - 1.f));
-                        const int qn = (int)ceilf(-fminf(fmaxf(v, 1.f - wa.scale), 0.f));
-                        const bool neg = qn > 0;
-                        const int mag = neg ? qn : qp;
-                        const uint32_t sw = lut_s[(neg ? row_off_neg : row_off_pos) + mag * WORDS + wd]; // row `value 0` is zero
-                        tile[cl * 32 + (lane ^ cl)] = reverse_nibbles(transpose32_warp(neg ? 0u : sw, lane));
-                        tile[1024 + cl * 32 + (lane ^ cl)] = reverse_nibbles(transpose32_warp(neg ? sw : 0u, lane));
+                    for (int k = 0; k < 8; k++) {
+                        const int c = b + k, at = (c & ~3) | (3 - (c & 3));
+                        const float x = wv[k] * wa.scale;
+                        // w_pos = ceil(clamp(x, 0, L-1)); w_neg = ceil(-clamp(x, 1-L, 0))  (sc_cuda.cpp:92-93): the
+                        // rounded magnitude of either sign, which only one of the two has
+                        const int mag = (int)ceilf(fminf(fabsf(x), wa.scale - 1.f));
+                        const bool neg = !(x >= 0.f); // (NaN: as the two clamps leave it)
+                        v[at] = lut_s[(neg ? pn : pp) * (uint32_t)row_words + (uint32_t)(mag * WORDS + wd)]; // row `value 0` is zero
+                        signs |= neg ? 1u << at : 0u;
+                        pp += seed_step;
+                        pn += seed_step;
+                        if (pp >= period) pp -= period;
+                        if (pn >= period) pn -= period;
                     }
                 }
-                __syncwarp();
+                transpose32_regs_prmt(v);
                 uint32_t *dst = Wb + (((size_t)nchunk * slots + wd * 32) * row_words_w + (size_t)tap * wa.CW + cw) * 128 + col0 + lane;
-#pragma unroll 4
+#pragma unroll
                 for (int sl = 0; sl < 32; sl++) {
-                    dst[0] = tile[lane * 32 + (sl ^ lane)];
-                    dst[64] = tile[1024 + lane * 32 + (sl ^ lane)];
+                    dst[0] = v[sl] & ~signs;
+                    dst[64] = v[sl] & signs;
                     dst += row_words_w * 128;
                 }
-                __syncwarp();
             }
         }
     }
     // (each warp goes on as soon as its own weight items are done: its staging area is its own)
-    expand_act_async_body<T, WORDS, NCHW>(a, x, lut_s, reinterpret_cast<uint8_t *>(lut_s) + lut_smem_bytes, 8192, sh, Ab, CW, n_groups);
+    expand_act_async_body<T, WORDS, NCHW>(a, x, lut_s, reinterpret_cast<uint8_t *>(lut_s) + lut_smem_bytes, 8192, sh, Ab, CW, n_groups, g.cw_parts);
 }
 
 template <typename T, int WORDS, bool NCHW>
-static int launch_expand_all_t(const ExpandAllArgs &g, const void *d_act, const void *d_w, uint32_t *d_Ab, uint32_t *d_Wb,
+static int launch_expand_all_t(ExpandAllArgs g, const void *d_act, const void *d_w, uint32_t *d_Ab, uint32_t *d_Wb,
                                int *d_status, int CW, size_t lut_bytes, cudaStream_t st)
 {
     const long long n_groups = (g.act.NHWp + 31) / 32;
     int dev = 0, sms = 0;
     REXSC_CUDA_CHECK(cudaGetDevice(&dev));
     REXSC_CUDA_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    long long blocks = (n_groups + kFastWarps - 1) / kFastWarps;
+    // Few pixel groups (small maps at small batches): share the channel words of a group out to several warps, up to as
+    // many as run at once; otherwise a warp keeps its group's pixel decode for all of them.
+    const long long warps = 2LL * sms * kFastWarps;
+    int parts = n_groups * 2 > warps ? 1 : (int)(warps / n_groups < CW ? warps / n_groups : CW);
+    parts = (CW + (CW + parts - 1) / parts - 1) / ((CW + parts - 1) / parts); // no part without words
+    g.cw_parts = parts;
+    long long blocks = (n_groups * parts + kFastWarps - 1) / kFastWarps;
     const long long wblocks = (g.w_items + kFastWarps - 1) / kFastWarps;
     if (blocks < wblocks) blocks = wblocks;
     if (blocks > 2LL * sms) blocks = 2LL * sms; // persistent: two CTAs per SM
@@ -1349,7 +1424,10 @@ int launch_expand_all_bits(const ConvPlan &p, const rexsc_sc_conv_desc &d, const
     g.lut = LutParams{p.l, d.bit_length, d.gen_config, xnor, d.prog_total_width, d.prog_load_width, d.prog_load_wait, p.words};
     g.w_dtype = d.w_dtype;
     g.w_items = (long long)w.NC * 2 * w.KHW * w.CW; // blocks of 32 output channels x taps x channel words
-    g.w_coarse = g.w_items >= 2048 ? 1 : 0;           // enough of them to occupy the grid's warps
+    // Blocks from about one per scheduler on: a block is some 1000 instructions for 32 x 32 weights, 32 single output
+    // channels are 2000, but there are 32 times as many warps to run them on.
+    g.w_coarse = g.w_items >= 512 ? 1 : 0;
+    g.w_vec = d.w_dtype == REXSC_F32 && d.w_channels_last && (p.C % 4) == 0 && (reinterpret_cast<uintptr_t>(d_w) & 15u) == 0 ? 1 : 0;
     if (!g.w_coarse) g.w_items *= 32;                 // single output channels
     if (opt.skip_weights) g.w_items = 0;
     g.verify_border = opt.verify_border ? 1 : 0;
@@ -1581,13 +1659,14 @@ __global__ void __launch_bounds__(256) expand_weight_bits_kernel(ExpandWBitsArgs
         const long long seed_ind = a.linear_seeds ? (long long)ci : ((long long)ci * a.KH + kh) * a.KW + kw;
         const int phase = (int)(((neg ? a.seed_neg : a.seed_pos) + seed_ind) % a.period);
         const int nchunk = co >> 6, col = co & 63;
+        const uint32_t signs = reverse_nibbles(__ballot_sync(0xffffffffu, neg));
         for (int wd = 0; wd < a.words; wd++) {
+            // a weight has one sign: the slot words of both signs are one transposed word under the sign mask
             const uint32_t v = mag > 0 ? __ldg(lut + ((size_t)phase * a.nvals + mag) * a.words + wd) : 0u;
-            const uint32_t tp = reverse_nibbles(transpose32_warp(neg ? 0u : v, lane));
-            const uint32_t tn = reverse_nibbles(transpose32_warp(neg ? v : 0u, lane));
+            const uint32_t tv = reverse_nibbles(transpose32_warp(v, lane));
             uint32_t *dst = Wb + (((size_t)nchunk * slots + wd * 32 + lane) * row_words + (size_t)tap * a.CW + cw) * 128 + col;
-            dst[0] = tp;
-            dst[64] = tn;
+            dst[0] = tv & ~signs;
+            dst[64] = tv & signs;
         }
     }
 }
