@@ -8,8 +8,9 @@
 // lanes), N = output-pixel candidates, K = taps x channels, issued as tcgen05.mma.kind::mxf4 M128 N160 K64.
 //
 // Why 4-bit floats.  0 and the powers of two that the operands use (0.5, 1, 2) are exact e2m1 numbers, every block
-// scale is 1, a coincidence contributes exactly 1.0 and fp32 accumulators count exactly to 2^24: the result is the
-// integer count.  Against the int8 kind the same channels take half the operand bytes and half the MMA time, and
+// scale is 1, a coincidence contributes exactly 1.0 and fp32 accumulators count exactly to 2^24.  One more MMA per unit
+// and slot starts the accumulators at 2^23, so that the low 16 bits of each ARE the integer count and a packed TMEM read
+// delivers two per register.  Against the int8 kind the same channels take half the operand bytes and half the MMA time, and
 // expanding 32 bits into 32 operands takes 5 logic instructions instead of 17.
 //
 // Why the weights are the TMEM operand.  The MMA reads its M operand from tensor memory and its N operand from shared
@@ -31,8 +32,8 @@
 //            to plane(kh % sh, kw % sw) + (kh / sh) * Wo + kw / sw rows: no im2col, for any stride.
 //   weights  the slot's weight bits, TMEM columns [tap][32-channel word][4 columns of 8 nibbles].
 //
-// Tensor memory (512 columns): two accumulator units of 160, two operand buffers of up to 72, 16 columns of block
-// scales (all 1, the same columns serve both operands).
+// Tensor memory (512 columns): two accumulator units of 160, two operand buffers of up to 72, 2 x 16 columns of block
+// scales (the same columns serve both operands), 8 of the bias MMA's weights.
 //
 // One persistent CTA per SM walks its tiles as a single pipeline (a tile's first loads and its store overlap the
 // neighbouring tiles' MMAs): eight warps fold counts, four expand operands, one issues the MMAs, unit 0 then unit 1 of
@@ -55,7 +56,7 @@ constexpr int kTcIssueWarp = kTcFoldWarps + kTcExpandWarps; // issues the MMAs
 constexpr int kTcLoadWarp = kTcIssueWarp + 1;               // copies the weight bit words into shared memory
 constexpr int kTcThreads = (kTcFoldWarps + kTcExpandWarps + 4) * 32; // whole warpgroups: two warps idle
 // Registers per thread: 896 threads are launched with 72, which the warpgroups share out again by what they need (the
-// folding warps hold 40 sum registers and 48 counts).
+// folding warps hold 40 sum and 40 count registers).
 constexpr int kTcRegsLaunch = 72, kTcRegsFold = 96, kTcRegsExpand = 40, kTcRegsIssuer = 32;
 static_assert(kTcFoldWarps * 32 * kTcRegsFold + kTcExpandWarps * 32 * kTcRegsExpand + 128 * kTcRegsIssuer <= kTcThreads * kTcRegsLaunch,
               "more registers than the block has");
@@ -71,8 +72,10 @@ constexpr int kTcMaxARows = 8;     // patch rows per expanding thread (all resid
 constexpr int kTcWordCols = 4;     // TMEM columns of one 32-channel weight word (8 nibbles per column)
 constexpr int kTcMaxWords = 18;    // weight words per row and step: the operand buffers' TMEM columns / kTcWordCols
 constexpr uint32_t kTcColA = 2 * kTcUnit;                                   // first column of the weight buffers
-constexpr uint32_t kTcColSf = kTcColA + 2 * kTcMaxWords * kTcWordCols;      // first column of the block scales
-static_assert(kTcColSf + 16 <= 512, "tensor memory has 512 columns");
+constexpr uint32_t kTcColSf = kTcColA + 2 * kTcMaxWords * kTcWordCols;      // block scales of the operands: 1
+constexpr uint32_t kTcColSfBias = kTcColSf + 16;                            // block scales of the bias MMA: 2^11
+constexpr uint32_t kTcColBias = kTcColSfBias + 16;                          // its weight operand: K element 0 is 2, the others 0
+static_assert(kTcColBias + 8 <= 512, "tensor memory has 512 columns");
 constexpr int kTcStageCols = 32;   // candidates that pass through a warp's store staging at a time
 constexpr int kTcStagePitch = kTcStageCols / 2 + 1; // words per row of a warp's store staging: odd, so rows change banks
 constexpr uint32_t kTcWaitLimit = 1u << 18; // try_wait attempts before a wait gives up (each may sleep kTcSuspendNs)
@@ -94,6 +97,7 @@ struct TcArgs {
     int tiles_x;       // candidate tiles = ceil(total_o / kTcM)
     int total_tiles;   // tiles_x * (64-channel output chunks); tile index = chunk * tiles_x + x
     int out_al4;       // both output pointers are 4-byte aligned: two channels of a pixel may be stored at once
+    int out_vec;       // ... 16-byte aligned, and so is every pixel's channel run: eight at once
     int balanced;      // 0: a CTA walks whole tiles blockIdx.x, + gridDim.x, ...
                        // 1: the (tile, time slot) pairs, in that order, are cut into gridDim.x equal runs, one per CTA.
                        //    A tile that two or more CTAs share is zeroed before the launch (zero_shared_tiles_kernel)
@@ -103,7 +107,6 @@ struct TcArgs {
                        //    channel runs): the host clears the whole outputs and every tile adds 16-bit values.
     long long NHWp;
     int out_nhwc;
-    int wide;        // 1: running sums (or the OR-n limit) exceed what fp16 counts exactly, so they are kept as integers
     int tap_off[kTcMaxTaps]; // patch-row offset of every tap (kernel parameters are warp-uniform by construction)
 };
 
@@ -150,18 +153,23 @@ __device__ __forceinline__ uint64_t desc_interleaved(uint32_t addr, uint32_t lbo
     return d;
 }
 
+// (a polling loop of four instructions: waiting warps share issue slots with working ones)
 __device__ __forceinline__ bool tc_wait(uint32_t bar, uint32_t parity)
 {
-    for (uint32_t i = 0; i < kTcWaitLimit; i++) {
-        uint32_t ok;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(ok) : "r"(bar), "r"(parity), "r"(kTcSuspendNs) : "memory");
-        if (ok) return true;
-    }
-    return false;
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t.reg .u32 left;\n\t"
+        "mov.u32 left, %4;\n"
+        "POLL_%=:\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+        "@p bra READY_%=;\n\t"
+        "sub.u32 left, left, 1;\n\t"
+        "setp.ne.u32 q, left, 0;\n\t"
+        "@q bra POLL_%=;\n"
+        "READY_%=:\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok) : "r"(bar), "r"(parity), "r"(kTcSuspendNs), "n"(kTcWaitLimit) : "memory");
+    return ok != 0;
 }
 
 // 32 bits -> 32 e2m1 operands (16 bytes).  A bit expands by masking where it stands: bits 0, 1, 2 of a nibble are the
@@ -178,13 +186,20 @@ __device__ __forceinline__ uint4 spread_weights(uint32_t h)
     return make_uint4(g & 0x44444444u, g & 0x22222222u, g & 0x11111111u, h & 0x11111111u);
 }
 
-#define REXSC_TMEM_LD16(arr, taddr)                                                                                   \
+// 32 (16) TMEM columns as 16 (8) registers: the low 16 bits of two adjacent columns per register
+#define REXSC_TMEM_LD32P(arr, taddr)                                                                                  \
     asm volatile(                                                                                                     \
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "                                                                     \
+        "tcgen05.ld.sync.aligned.32x32b.x16.pack::16b.b32 "                                                           \
         "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"                              \
         : "=r"(arr[0]), "=r"(arr[1]), "=r"(arr[2]), "=r"(arr[3]), "=r"(arr[4]), "=r"(arr[5]), "=r"(arr[6]),           \
           "=r"(arr[7]), "=r"(arr[8]), "=r"(arr[9]), "=r"(arr[10]), "=r"(arr[11]), "=r"(arr[12]), "=r"(arr[13]),       \
           "=r"(arr[14]), "=r"(arr[15])                                                                                \
+        : "r"(taddr)                                                                                                  \
+        : "memory")
+#define REXSC_TMEM_LD16P(arr, taddr)                                                                                  \
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.pack::16b.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"            \
+        : "=r"(arr[0]), "=r"(arr[1]), "=r"(arr[2]), "=r"(arr[3]), "=r"(arr[4]), "=r"(arr[5]), "=r"(arr[6]),           \
+          "=r"(arr[7])                                                                                                \
         : "r"(taddr)                                                                                                  \
         : "memory")
 
@@ -195,18 +210,26 @@ __device__ __forceinline__ uint4 spread_weights(uint32_t h)
           "+r"(arr[7]), "+r"(arr[8]), "+r"(arr[9]), "+r"(arr[10]), "+r"(arr[11]), "+r"(arr[12]), "+r"(arr[13]),       \
           "+r"(arr[14]), "+r"(arr[15])                                                                                \
         :: "memory")
+#define REXSC_TMEM_WAIT8(arr)                                                                                         \
+    asm volatile("tcgen05.wait::ld.sync.aligned;"                                                                     \
+        : "+r"(arr[0]), "+r"(arr[1]), "+r"(arr[2]), "+r"(arr[3]), "+r"(arr[4]), "+r"(arr[5]), "+r"(arr[6]),           \
+          "+r"(arr[7])                                                                                                \
+        :: "memory")
+
 // KHW_T: taps known at compile time (9, 1) or 0 for any tap count up to kTcMaxTaps
 // KWC:   32-channel words per pipeline step (TcArgs::KWc; above 4 only with KHW_T == 1)
 // RA:    patch rows per expanding thread (1 .. kTcMaxARows)
 //
 // What bounds it, and the split of the warps.  The MMAs of a step take 18 x 83 clk on a 3x3 layer; everything else has
-// to fit beside them.  Folding costs three instructions per two counts (convert, minimum, add; the first two on the ALU,
-// at half rate) and expanding five per 32 operands, so the instruction count decides, and with it what every warp
-// repeats per step: addresses, waits, hand-overs.  Measured on 64 -> 64 channels, 3x3, 56x56, 32 slots, batch 256 (whole
-// call; tensor pipe busy): int8 operands, both in shared memory, 16 warps on both jobs 1.13 ms (80 % of an int8 pipe of
-// half the rate); 4-bit with 16 such warps 1.32 ms (43 %); 8 folding + 4 expanding warps 0.95 ms; 8 + 8 with the weight
-// words brought in by bulk copies 1.01 ms (48 %; the folding warps waited for five TMEM reads per unit, one after the
-// other); 16 folding warps, eight per unit, + 8 expanding: 0.84 ms.  512 -> 512 channels, 7x7: 1.19 -> 0.69 ms (87 %).
+// to fit beside them, so the instruction count decides, and with it what every warp repeats per step: addresses, waits,
+// hand-overs.  Measured on 64 -> 64 channels, 3x3, 56x56, 32 slots, batch 256 (accumulate launch alone; tensor pipe busy):
+//   int8 operands, both in shared memory, 16 warps on both jobs            1.02 ms (80 % of an int8 pipe of half the rate)
+//   4-bit, 16 such warps                                                    1.20 ms (43 %)
+//   8 folding + 4 expanding warps                                           0.83 ms
+//   16 folding (eight per unit) + 8 expanding, fp32 counts read in two goes 0.74 ms (59 %)
+//   2^23 bias: packed counts, one read per unit and slot; 16-byte stores    0.64 ms
+// of which the MMAs are 0.54 ms.  512 -> 512 channels, 7x7: 1.13 -> 0.60 ms, the MMAs alone.  1x1 filters on few channels
+// stay bound by the hand-overs of a slot (MMA, commit, TMEM read, release: some 1600 clk for both units).
 template <int KHW_T, int KWC, int RA>
 __global__ void __launch_bounds__(kTcThreads, 1)
 sc_conv_tc_kernel(TcArgs a, const uint32_t *__restrict__ Ab, const uint32_t *__restrict__ Wb,
@@ -224,7 +247,8 @@ sc_conv_tc_kernel(TcArgs a, const uint32_t *__restrict__ Ab, const uint32_t *__r
     uint32_t *stage_all = reinterpret_cast<uint32_t *>(smem + 2 * a_bytes); // [fold warp][32 rows][kTcStagePitch]
     uint32_t *w_ring = stage_all + kTcFoldWarps * 32 * kTcStagePitch;       // [depth][tap][KWC][kTcN] weight bit words
     uint32_t *p_ring = w_ring + a.depth * (KHW * KWC * kTcN);               // [depth][RA][KWC][256] patch bit words
-    uint64_t *bars = reinterpret_cast<uint64_t *>(p_ring + a.depth * (RA * KWC * kTcExpandWarps * 32));
+    uint4 *bias_s = reinterpret_cast<uint4 *>(p_ring + a.depth * (RA * KWC * kTcExpandWarps * 32)); // [2][kTcUnit] pixel operand of 1s
+    uint64_t *bars = reinterpret_cast<uint64_t *>(bias_s + 2 * kTcUnit);
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + kTcBars);
 
     const int tid = threadIdx.x, lane = tid & 31;
@@ -288,13 +312,23 @@ sc_conv_tc_kernel(TcArgs a, const uint32_t *__restrict__ Ab, const uint32_t *__r
     const uint32_t tmem_base = *tmem_slot;
     const uint32_t lane_quarter = (uint32_t)((warp & 3) * 32) << 16; // the TMEM lanes this warp can access
     if (warp < 4) {
-        // block scales: 2^0 (biased exponent 127) in every byte, whatever row or block an MMA reads from them
-        const uint32_t one = 0x7f7f7f7fu;
-        asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
-                     "{%1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1};" ::"r"(tmem_base + kTcColSf + lane_quarter),
-                     "r"(one) : "memory");
+        // block scales (biased exponents, the same in every byte, whatever row or block an MMA reads) and the weight
+        // operand of the bias MMA
+        auto fill = [&](uint32_t col, uint32_t v) {
+            asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %1, %1, %1, %1, %1, %1, %1};"
+                         ::"r"(tmem_base + lane_quarter + col), "r"(v) : "memory");
+        };
+        fill(kTcColSf, 0x7f7f7f7fu);
+        fill(kTcColSf + 8, 0x7f7f7f7fu);
+        fill(kTcColSfBias, 0x8a8a8a8au);
+        fill(kTcColSfBias + 8, 0x8a8a8a8au);
+        const uint32_t z = 0u, two = 4u; // e2m1 2.0 in the lowest nibble
+        asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %2, %2, %2, %2, %2, %2};"
+                     ::"r"(tmem_base + lane_quarter + kTcColBias), "r"(two), "r"(z) : "memory");
         asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
     }
+    for (int i = tid; i < 2 * kTcUnit; i += kTcThreads) bias_s[i] = make_uint4(0x22222222u, 0x22222222u, 0x22222222u, 0x22222222u);
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -330,6 +364,7 @@ sc_conv_tc_kernel(TcArgs a, const uint32_t *__restrict__ Ab, const uint32_t *__r
         for (int tap = 0; tap < kTcMaxTaps; tap++) p_tap[tap] = tap < KHW ? (uint32_t)a.tap_off[tap] : 0u;
         const uint64_t dp_proto = desc_interleaved(saddr(smem), (uint32_t)a.rows_a * 16);
         const uint32_t dp_hi = (uint32_t)(dp_proto >> 32);
+        const uint64_t db_bias = desc_interleaved(saddr(bias_s), kTcUnit * 16);
         const uint32_t sf = tmem_base + kTcColSf;
         auto commit = [&](uint64_t *bar) { // arrives on the barrier when every MMA issued so far has completed
             asm volatile("{\n\t.reg .pred e;\n\telect.sync _|e, 0xffffffff;\n\t"
@@ -341,7 +376,18 @@ sc_conv_tc_kernel(TcArgs a, const uint32_t *__restrict__ Ab, const uint32_t *__r
             const uint32_t w_lo = tmem_base + kTcColA + (uint32_t)(buf * kTcMaxWords * kTcWordCols);
             const uint32_t d_addr = tmem_base + (uint32_t)(u * kTcUnit);
             const int words = a.CW - ck * KWC; // words left in this chunk; an odd last one is paired with a zero word
-            const uint32_t first_acc = ck > 0 ? 1u : 0u;
+            auto mma = [&](uint32_t wcol, uint32_t plo, uint32_t phi, uint32_t scales, uint32_t accumulate) {
+                asm volatile(
+                    "{\n\t.reg .pred p, e;\n\t.reg .b64 db;\n\t"
+                    "mov.b64 db, {%2, %3};\n\t"
+                    "setp.ne.b32 p, %5, 0;\n\t"
+                    "elect.sync _|e, 0xffffffff;\n\t"
+                    "@e tcgen05.mma.cta_group::1.kind::mxf4.block_scale.scale_vec::2X [%0], [%1], db, %4, [%6], [%6], p;\n\t}"
+                    ::"r"(d_addr), "r"(wcol), "r"(plo), "r"(phi), "r"(idesc), "r"(accumulate), "r"(scales)
+                    : "memory");
+            };
+            // a slot starts at 2^23 = (1 * 2^11) * (2 * 2^11): the counts then are the low bits of the accumulators
+            if (ck == 0) mma(tmem_base + kTcColBias, (uint32_t)db_bias, (uint32_t)(db_bias >> 32), tmem_base + kTcColSfBias, 0u);
 #pragma unroll
             for (int tap = 0; tap < (KHW_T ? KHW_T : kTcMaxTaps); tap++) {
                 if (KHW_T || tap < a.KHW) {
@@ -350,15 +396,7 @@ sc_conv_tc_kernel(TcArgs a, const uint32_t *__restrict__ Ab, const uint32_t *__r
                         if (k > 0 && k >= words) break;
                         const uint32_t plo = dp_lo + p_tap[tap] + (uint32_t)k * (uint32_t)a.rows_a;
                         const uint32_t wcol = w_lo + (uint32_t)((tap * KWC + k) * kTcWordCols);
-                        const uint32_t accumulate = (tap > 0 || k > 0) ? 1u : first_acc;
-                        asm volatile(
-                            "{\n\t.reg .pred p, e;\n\t.reg .b64 db;\n\t"
-                            "mov.b64 db, {%2, %3};\n\t"
-                            "setp.ne.b32 p, %5, 0;\n\t"
-                            "elect.sync _|e, 0xffffffff;\n\t"
-                            "@e tcgen05.mma.cta_group::1.kind::mxf4.block_scale.scale_vec::2X [%0], [%1], db, %4, [%6], [%6], p;\n\t}"
-                            ::"r"(d_addr), "r"(wcol), "r"(plo), "r"(dp_hi), "r"(idesc), "r"(accumulate), "r"(sf)
-                            : "memory");
+                        mma(wcol, plo, dp_hi, sf, 1u);
                     }
                 }
             }
@@ -539,59 +577,34 @@ sc_conv_tc_kernel(TcArgs a, const uint32_t *__restrict__ Ab, const uint32_t *__r
         // ---- folding warps: counts -> min(count, n) -> running sums -> outputs ----
         asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kTcRegsFold));
         // Warps 0-7 fold unit 0 while the tensor core is on unit 1, warps 8-15 the other way round.  This thread owns one
-        // weight row (lane 32*(warp%4)+lane = sign and output channel) and kTcCols candidates of its unit; two running
-        // sums per register: fp16 (exact up to 2048) or, where they can be larger, 16-bit integers.
+        // weight row (lane 32*(warp%4)+lane = sign and output channel) and kTcCols candidates of its unit, two 16-bit
+        // sums per register.
         uint32_t sum[kTcCols / 2];
 #pragma unroll
         for (int j = 0; j < kTcCols / 2; j++) sum[j] = 0u;
         const int u = warp >> 3, col0 = ((warp >> 2) & 1) * kTcCols; // unit, first column of the warp in it
         const uint32_t taddr = tmem_base + lane_quarter + (uint32_t)(u * kTcUnit + col0);
-        // fp16: the conversion rounds counts above 2048, which keeps them above every n it is used with; conversion,
-        // minimum and addition take one instruction per two counts.
-        const __half2 n2h = __half2half2(__int2half_rn(a.wide ? 0 : a.n_or));
-        const uint32_t n2i = (uint32_t)a.n_or * 0x00010001u;
-        auto add16 = [&](uint32_t *sum8, const uint32_t (&x)[16]) {
-            if (!a.wide) {
-#pragma unroll
-                for (int j = 0; j < 8; j++) {
-                    const __half2 cnt = __floats2half2_rn(__uint_as_float(x[2 * j]), __uint_as_float(x[2 * j + 1]));
-                    __half2 t = *reinterpret_cast<__half2 *>(&sum8[j]);
-                    t = __hadd2(t, __hmin2(cnt, n2h));
-                    sum8[j] = *reinterpret_cast<uint32_t *>(&t);
-                }
-            } else { // + 2^23 puts the integer into the low bits of the float
-#pragma unroll
-                for (int j = 0; j < 8; j++) {
-                    const uint32_t cnt = __byte_perm(__float_as_uint(__uint_as_float(x[2 * j]) + 8388608.0f),
-                                                     __float_as_uint(__uint_as_float(x[2 * j + 1]) + 8388608.0f), 0x5410);
-                    sum8[j] += __vminu2(cnt, n2i);
-                }
-            }
-        };
-        // A TMEM read takes some 250 clk while MMAs run, so few reads are waited for: 48 columns, then 32 whose latency
-        // the arithmetic on the first ones covers.
+        const uint32_t n2 = (uint32_t)a.n_or * 0x00010001u;
+        // The accumulators are 2^23 + count, so the packed read delivers two integer counts per register.  All of them
+        // are read at once and handed back before the arithmetic: the unit's next MMAs wait for one TMEM read.
         auto fold_slot = [&]() {
-            uint32_t x0[16], x1[16], x2[16];
-            REXSC_TMEM_LD16(x0, taddr);
-            REXSC_TMEM_LD16(x1, taddr + 16u);
-            REXSC_TMEM_LD16(x2, taddr + 32u);
+            uint32_t x0[16], x1[16], x2[8];
+            REXSC_TMEM_LD32P(x0, taddr);
+            REXSC_TMEM_LD32P(x1, taddr + 32u);
+            REXSC_TMEM_LD16P(x2, taddr + 64u);
             REXSC_TMEM_WAIT16(x0);
             REXSC_TMEM_WAIT16(x1);
-            REXSC_TMEM_WAIT16(x2);
-            add16(sum, x0);
-            REXSC_TMEM_LD16(x0, taddr + 48u);
-            add16(sum + 8, x1);
-            REXSC_TMEM_LD16(x1, taddr + 64u);
-            add16(sum + 16, x2);
-            REXSC_TMEM_WAIT16(x0);
-            REXSC_TMEM_WAIT16(x1);
-            // the last counts are in registers: hand the accumulators back
+            REXSC_TMEM_WAIT8(x2);
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             warp_arrive(&bar_tfree[u]);
-            add16(sum + 24, x0);
-            add16(sum + 32, x1);
+#pragma unroll
+            for (int j = 0; j < 16; j++) sum[j] += __vminu2(x0[j], n2);
+#pragma unroll
+            for (int j = 0; j < 16; j++) sum[16 + j] += __vminu2(x1[j], n2);
+#pragma unroll
+            for (int j = 0; j < 8; j++) sum[32 + j] += __vminu2(x2[j], n2);
         };
-        static_assert(kTcCols == 80, "fold_slot reads 5 x 16 columns");
+        static_assert(kTcCols == 80, "fold_slot reads 32 + 32 + 16 columns");
         // Running sums -> int16 outputs, after the last slot of tile k.  A warp holds 32 output channels of one sign x
         // kTcCols candidates; they pass through its staging rows, 32 at a time, so that stores run along channels
         // (channels_last) or along pixels (channel-planar).  A candidate (i, j) of the origin grid is an output pixel
@@ -615,12 +628,7 @@ sc_conv_tc_kernel(TcArgs a, const uint32_t *__restrict__ Ab, const uint32_t *__r
 #pragma unroll
                 for (int j = 0; j < kS / 2; j++) {
                     if (h / 2 + j >= kTcCols / 2) break;
-                    uint32_t v = sum[h / 2 + j];
-                    if (!a.wide) {
-                        const __half2 t = *reinterpret_cast<const __half2 *>(&v);
-                        v = (uint32_t)__half2ushort_rn(__low2half(t)) | ((uint32_t)__half2ushort_rn(__high2half(t)) << 16);
-                    }
-                    stage[lane * kTcStagePitch + j] = v;
+                    stage[lane * kTcStagePitch + j] = sum[h / 2 + j];
                     sum[h / 2 + j] = 0u;
                 }
                 __syncwarp();
@@ -635,11 +643,25 @@ sc_conv_tc_kernel(TcArgs a, const uint32_t *__restrict__ Ab, const uint32_t *__r
                         base = (long long)(a.out_nhwc ? ((size_t)n * ohw + pix) * a.Co : (size_t)n * a.Co * ohw + pix);
                     }
                 }
-                if (a.balanced != 2 && a.out_nhwc && a.out_al4 && (a.Co & 1) == 0) {
+                if (a.balanced != 2 && a.out_nhwc && a.out_vec && !shared_tile) {
+                    // eight channels per lane, eight pixels at a time
+                    const int c8 = (lane & 3) * 8;
+#pragma unroll 2
+                    for (int p = lane >> 2; p < cnt; p += 8) {
+                        const long long b = __shfl_sync(0xffffffffu, base, p);
+                        uint32_t v[4];
+#pragma unroll
+                        for (int q = 0; q < 4; q++)
+                            v[q] = (uint32_t)stage16[(c8 + 2 * q) * (2 * kTcStagePitch) + p] |
+                                   ((uint32_t)stage16[(c8 + 2 * q + 1) * (2 * kTcStagePitch) + p] << 16);
+                        if (b >= 0 && co0 + c8 < a.Co)
+                            *reinterpret_cast<uint4 *>(dst + b + co0 + c8) = make_uint4(v[0], v[1], v[2], v[3]);
+                    }
+                } else if (a.balanced != 2 && a.out_nhwc && a.out_al4 && (a.Co & 1) == 0) {
                     // two channels per lane, two pixels per store
-                    const int w = lane & 15, hp = lane >> 4;
+                    const int w = lane & 15;
 #pragma unroll 4
-                    for (int p = hp; p < cnt; p += 2) {
+                    for (int p = lane >> 4; p < cnt; p += 2) {
                         const long long b = __shfl_sync(0xffffffffu, base, p);
                         if (b >= 0 && co0 + 2 * w < a.Co) {
                             const uint32_t v = (uint32_t)stage16[(2 * w) * (2 * kTcStagePitch) + p] |
@@ -796,8 +818,8 @@ __global__ void __launch_bounds__(128, 2) mma_probe_kernel(int iters, int n_cols
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    uint32_t v[16];
-    REXSC_TMEM_LD16(v, tmem_base + ((uint32_t)(warp * 32) << 16));
+    uint32_t v[8];
+    REXSC_TMEM_LD16P(v, tmem_base + ((uint32_t)(warp * 32) << 16));
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
     sink[blockIdx.x * blockDim.x + tid] = v[0] + (ok ? 0u : 0x80000000u);
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -847,7 +869,8 @@ TcGeom tc_geometry(const ConvPlan &p)
     g.ra = p.KHW == 1 || g.ra <= 2 ? 2 : g.ra <= 6 ? 6 : kTcMaxARows; // the instantiated row counts
     auto need = [&](int depth) {
         return 2 * (size_t)g.KWc * g.rows_a * 16 + (size_t)kTcFoldWarps * 32 * kTcStagePitch * 4 +
-               (size_t)depth * g.KWc * 4 * (p.KHW * kTcN + g.ra * kTcExpandWarps * 32) + kTcBars * 8 + 8 + sizeof(TileRun) + 128;
+               (size_t)depth * g.KWc * 4 * (p.KHW * kTcN + g.ra * kTcExpandWarps * 32) + 2 * kTcUnit * 16 + kTcBars * 8 + 8 +
+               sizeof(TileRun) + 128;
     };
     g.depth = need(kTcMaxDepth) <= 227 * 1024 ? kTcMaxDepth : 2;
     if (need(g.depth) > 227 * 1024) return g;
@@ -979,9 +1002,9 @@ int launch_conv_tc(const ConvPlan &p, const rexsc_sc_conv_desc &d, void *d_tc_ws
     a.NHWp = p.NHWp; a.out_nhwc = d.out_channels_last;
     if ((reinterpret_cast<uintptr_t>(d_pos) | reinterpret_cast<uintptr_t>(d_neg)) & 1u) return REXSC_E_BAD_ARG;
     a.out_al4 = aligned4 ? 1 : 0;
+    a.out_vec = ((reinterpret_cast<uintptr_t>(d_pos) | reinterpret_cast<uintptr_t>(d_neg)) & 15u) == 0 && (p.Co & 7) == 0 ? 1 : 0;
     {
         const long long cap = p.n_or < p.Kdot ? p.n_or : p.Kdot;
-        a.wide = (long long)slots * cap > 2048 ? 1 : 0; // fp16 counts exactly up to 2048
         a.n_or = (int)cap; // a count never exceeds the dot length, so clamping there changes nothing
     }
     for (int t = 0; t < kTcMaxTaps; t++) a.tap_off[t] = g.tap_off[t];
