@@ -77,9 +77,12 @@ static int grid_mode(const rexsc_sc_conv_desc *desc, const ConvPlan &p, int kern
 // stage 1: stream generation (LUTs, activation words, weight words + signs) into the workspace.
 // allow_partial: a null operand is skipped and what an earlier expand with the same descriptor and workspace wrote
 // for it stays in place (a caller whose weights do not change between calls expands them once).
+// d_out_*, outputs_cleared: with outputs at hand (the accumulate stage follows on the same stream) the stage also clears
+// them where that stage would have to, and says so.
 static int conv_expand(const rexsc_sc_conv_desc *desc, const void *d_act, const void *d_weight, void *d_workspace,
                        size_t workspace_bytes, cudaStream_t st, bool allow_partial, int w_seed_pos = 13,
-                       int w_seed_neg = 13)
+                       int w_seed_neg = 13, int16_t *d_out_pos = nullptr, int16_t *d_out_neg = nullptr,
+                       bool *outputs_cleared = nullptr)
 {
     ConvPlan p, pc;
     ConvBuffers b;
@@ -103,14 +106,19 @@ static int conv_expand(const rexsc_sc_conv_desc *desc, const void *d_act, const 
         const bool no_w = d_weight == nullptr;
         if (mode == kGridSpeculative) {
             REXSC_CUDA_CHECK(cudaMemsetAsync(b.status, 0, 256, st));
+            // (cleared for the launch on the compact grid; the one on the standard grid stores whole tiles)
+            const long long clear = outputs_cleared ? conv_tc_clear_words(pc, *desc, d_out_pos, d_out_neg) : 0;
             rc = launch_expand_all_bits(pc, *desc, d_act, d_weight, xnor, Ab, Wb, b.status,
-                                        ExpandAllOptions{true, false, no_w}, st);
+                                        ExpandAllOptions{true, false, no_w, {d_out_pos, d_out_neg}, clear}, st);
+            if (rc == REXSC_OK && clear > 0) *outputs_cleared = true;
             if (rc == REXSC_OK) // the standard planes, if the border turned out not to be zero
                 rc = launch_expand_all_bits(p, *desc, d_act, d_weight, xnor, Ab, Wb, b.status,
-                                            ExpandAllOptions{false, true, true}, st);
+                                            ExpandAllOptions{false, true, true, {nullptr, nullptr}, 0}, st);
         } else {
+            const long long clear = outputs_cleared ? conv_tc_clear_words(pa, *desc, d_out_pos, d_out_neg) : 0;
             rc = launch_expand_all_bits(pa, *desc, d_act, d_weight, xnor, Ab, Wb, b.status,
-                                        ExpandAllOptions{false, false, no_w}, st);
+                                        ExpandAllOptions{false, false, no_w, {d_out_pos, d_out_neg}, clear}, st);
+            if (rc == REXSC_OK && clear > 0) *outputs_cleared = true;
         }
         if (rc != REXSC_E_UNSUPPORTED) return rc;
     }
@@ -145,7 +153,7 @@ static int conv_expand(const rexsc_sc_conv_desc *desc, const void *d_act, const 
 
 // stage 2: OR-n accumulation over the stream words of the workspace
 static int conv_accumulate(const rexsc_sc_conv_desc *desc, int16_t *d_out_pos, int16_t *d_out_neg,
-                           void *d_workspace, size_t workspace_bytes, cudaStream_t st)
+                           void *d_workspace, size_t workspace_bytes, cudaStream_t st, bool outputs_cleared = false)
 {
     ConvPlan p, pc;
     ConvBuffers b;
@@ -157,12 +165,13 @@ static int conv_accumulate(const rexsc_sc_conv_desc *desc, int16_t *d_out_pos, i
     if (k == REXSC_KERNEL_TENSOR) {
         const size_t w_off = conv_tc_weight_offset(p);
         const int mode = grid_mode(desc, p, k, &pc);
-        if (mode == kGridStandard) return launch_conv_tc(p, *desc, b.tc, w_off, d_out_pos, d_out_neg, b.status, 0, st);
-        if (mode == kGridCompact) return launch_conv_tc(pc, *desc, b.tc, w_off, d_out_pos, d_out_neg, b.status, 0, st);
+        if (mode != kGridSpeculative)
+            return launch_conv_tc(mode == kGridCompact ? pc : p, *desc, b.tc, w_off, d_out_pos, d_out_neg, b.status, 0,
+                                  outputs_cleared, st);
         // one launch per possible verdict of the expand stage
-        rc = launch_conv_tc(pc, *desc, b.tc, w_off, d_out_pos, d_out_neg, b.status, +1, st);
+        rc = launch_conv_tc(pc, *desc, b.tc, w_off, d_out_pos, d_out_neg, b.status, +1, outputs_cleared, st);
         if (rc != REXSC_OK) return rc;
-        return launch_conv_tc(p, *desc, b.tc, w_off, d_out_pos, d_out_neg, b.status, -1, st);
+        return launch_conv_tc(p, *desc, b.tc, w_off, d_out_pos, d_out_neg, b.status, -1, false, st);
     }
     if (k == REXSC_KERNEL_TILED)
         return launch_conv_tiled(p, *desc, b.A, b.Wt, b.S, d_out_pos, d_out_neg, b.status, st);
@@ -178,9 +187,11 @@ int conv_forward(const rexsc_sc_conv_desc *desc, const void *d_act, const void *
         int rc = make_conv_plan(desc, &p);
         return rc != REXSC_OK ? rc : REXSC_E_BAD_ARG;
     }
-    int rc = conv_expand(desc, d_act, d_weight, d_workspace, workspace_bytes, st, false, w_seed_pos, w_seed_neg);
+    bool cleared = false;
+    int rc = conv_expand(desc, d_act, d_weight, d_workspace, workspace_bytes, st, false, w_seed_pos, w_seed_neg, d_out_pos,
+                         d_out_neg, &cleared);
     if (rc != REXSC_OK) return rc;
-    return conv_accumulate(desc, d_out_pos, d_out_neg, d_workspace, workspace_bytes, st);
+    return conv_accumulate(desc, d_out_pos, d_out_neg, d_workspace, workspace_bytes, st, cleared);
 }
 
 static void linear_desc(rexsc_sc_conv_desc *d, int32_t batch, int32_t c_in, int32_t c_out, int32_t act_dtype,

@@ -158,13 +158,19 @@ size_t conv_tc_weight_offset(const ConvPlan &p);
 //   otherwise (the caller clears the status block before the launch; the kernel then leaves it alone);
 // opt.gate: run only if d_status[1] != 0 (the fallback launch after a failed verification);
 // opt.skip_weights: activations only.
-struct ExpandAllOptions { bool verify_border, gate, skip_weights; };
+// opt.clear: two arrays of clear_n 16-byte words that the kernel also sets to zero (the outputs of a conv launch that adds
+//   into them).
+struct ExpandAllOptions { bool verify_border, gate, skip_weights; void *clear[2]; long long clear_n; };
 int launch_expand_all_bits(const ConvPlan &p, const rexsc_sc_conv_desc &d, const void *d_act, const void *d_w, int xnor,
                            uint32_t *d_Ab, uint32_t *d_Wb, int *d_status, const ExpandAllOptions &opt, cudaStream_t st);
 // gate: 0 = run always; +1 = run only if d_status[1] == 0 (compact planes valid); -1 = only if d_status[1] != 0.
 // weight_offset: byte offset of the weight bit planes in d_tc_ws (that of the standard plan, whatever grid p has).
+// outputs_cleared: the outputs are zero already (see conv_tc_clear_words).
 int launch_conv_tc(const ConvPlan &p, const rexsc_sc_conv_desc &d, void *d_tc_ws, size_t weight_offset, int16_t *d_pos,
-                   int16_t *d_neg, int *d_status, int gate, cudaStream_t st);
+                   int16_t *d_neg, int *d_status, int gate, bool outputs_cleared, cudaStream_t st);
+// 16-byte words per output tensor that the expand launch may as well clear for an ungated launch_conv_tc: 0 when that
+// launch stores whole tiles, or when clearing whole outputs would cost more than clearing the shared tiles does.
+long long conv_tc_clear_words(const ConvPlan &p, const rexsc_sc_conv_desc &d, const int16_t *d_pos, const int16_t *d_neg);
 
 // ---- device helpers -----------------------------------------------------------------------
 template <typename T> __device__ __forceinline__ float load_as_float(const T *p, long long i);

@@ -931,8 +931,59 @@ static int device_sms(int *sms)
     return REXSC_OK;
 }
 
+// One persistent CTA per SM (the kernel owns the SM's tensor memory).  Whole tiles dealt round-robin leave SMs idle in
+// the last wave (900 tiles on 148 SMs: 7 waves for the work of 6.1); cutting the (tile, slot) sequence into equal runs
+// does not.  balanced: see TcArgs.
+struct TcSplit { int balanced; unsigned grid; };
+
+static TcSplit tc_split(const ConvPlan &p, const rexsc_sc_conv_desc &d, const int16_t *d_pos, const int16_t *d_neg, int gate,
+                        int sms, long long total_tiles)
+{
+    TcSplit r{0, (unsigned)(total_tiles < sms ? total_tiles : sms)};
+    static const bool allow_balanced = !(getenv("REXSC_TC_BALANCED") && getenv("REXSC_TC_BALANCED")[0] == '0');
+    // The cut tiles are summed with packed 32-bit atomic adds, which need 4-byte aligned rows of whole 64-channel chunks;
+    // the fallback launch of a gated pair keeps whole tiles (it is the rare one and a second clearing kernel would cost
+    // every call).
+    const bool aligned4 = ((reinterpret_cast<uintptr_t>(d_pos) | reinterpret_cast<uintptr_t>(d_neg)) & 3u) == 0;
+    const bool rows_ok = d.out_channels_last && (p.Co % kTcCout) == 0 && aligned4;
+    // (measured: tiles with little tensor work per slot -- 1x1 filters on up to 256 channels -- gain nothing: their
+    // time goes to the per-slot hand-offs, and the atomic stores of the cut tiles cost more than the idle SMs did)
+    const bool heavy_slots = p.KHW * ((p.C + 31) / 32) >= 16 || total_tiles < sms;
+    if (!allow_balanced || !heavy_slots || !aligned4 || gate < 0 || total_tiles % sms == 0) return r;
+    // Outputs without such rows (NCHW, a ragged last chunk): clear them whole and let every tile add single 16-bit
+    // values -- affordable while the outputs are small, which is where whole tiles waste most (deep layers with few
+    // tiles per SM).  The element count must be even so that the last value's 32-bit word ends inside the tensor.
+    const size_t out_elems = (size_t)p.M * p.Co;
+    if (!rows_ok && ((out_elems & 1) != 0 || out_elems * sizeof(int16_t) > ((size_t)16 << 20))) return r;
+    // short layers: as many CTAs as leaves each about four slots to amortise its prologue
+    long long ctas = total_tiles * p.words * 32 / 4;
+    if (ctas < 1) ctas = 1;
+    if (ctas > sms) ctas = sms;
+    // worth a clearing launch when the last wave of whole tiles would waste more than 1 % (single values: 5 %) of the SM time
+    const long long waves = (total_tiles + sms - 1) / sms;
+    if ((double)total_tiles / sms < (rows_ok ? 0.99 : 0.95) * (double)waves || ctas > (long long)r.grid) {
+        r.balanced = rows_ok ? 1 : 2;
+        r.grid = (unsigned)ctas;
+    }
+    return r;
+}
+
+long long conv_tc_clear_words(const ConvPlan &p, const rexsc_sc_conv_desc &d, const int16_t *d_pos, const int16_t *d_neg)
+{
+    const size_t bytes = (size_t)p.M * p.Co * sizeof(int16_t);
+    // 4 MB per sign are about 1 us of the expand launch; clearing the shared tiles alone is a launch of 4 us
+    if (bytes > ((size_t)4 << 20) || (bytes & 15) != 0) return 0;
+    if ((reinterpret_cast<uintptr_t>(d_pos) | reinterpret_cast<uintptr_t>(d_neg)) & 15u) return 0;
+    int sms = 0;
+    if (!conv_tc_supported(p) || device_sms(&sms) != REXSC_OK) return 0;
+    const TcGeom g = tc_geometry(p);
+    const long long tiles_x = ((long long)p.N * g.Ho * g.Wo + kTcM - 1) / kTcM;
+    const TcSplit r = tc_split(p, d, d_pos, d_neg, 0, sms, tiles_x * ((p.Co + kTcCout - 1) / kTcCout));
+    return r.balanced ? (long long)(bytes / 16) : 0;
+}
+
 int launch_conv_tc(const ConvPlan &p, const rexsc_sc_conv_desc &d, void *d_tc_ws, size_t weight_offset, int16_t *d_pos,
-                   int16_t *d_neg, int *d_status, int gate, cudaStream_t st)
+                   int16_t *d_neg, int *d_status, int gate, bool outputs_cleared, cudaStream_t st)
 {
     if (!conv_tc_supported(p)) return REXSC_E_UNSUPPORTED;
     const TcGeom g = tc_geometry(p);
@@ -952,50 +1003,16 @@ int launch_conv_tc(const ConvPlan &p, const rexsc_sc_conv_desc &d, void *d_tc_ws
     int sms = 0;
     if (int rc = device_sms(&sms)) return rc;
     a.total_tiles = a.tiles_x * NC;
-    // One persistent CTA per SM (the kernel owns the SM's tensor memory).  Whole tiles dealt round-robin leave SMs idle
-    // in the last wave (900 tiles on 148 SMs: 7 waves for the work of 6.1); cutting the (tile, slot) sequence into
-    // equal runs does not.  The cut tiles are summed with packed 32-bit atomic adds, which need 4-byte aligned rows
-    // of whole 64-channel chunks; the fallback launch of a gated pair keeps whole tiles (it is the rare one and a
-    // second clearing kernel would cost every call).
-    const long long units = (long long)a.total_tiles * slots;
     const bool aligned4 = ((reinterpret_cast<uintptr_t>(d_pos) | reinterpret_cast<uintptr_t>(d_neg)) & 3u) == 0;
-    const bool rows_ok = d.out_channels_last && (p.Co % kTcCout) == 0 && aligned4;
-    unsigned grid = (unsigned)(a.total_tiles < sms ? a.total_tiles : sms);
-    a.balanced = 0;
-    static const bool allow_balanced = !(getenv("REXSC_TC_BALANCED") && getenv("REXSC_TC_BALANCED")[0] == '0');
-    // (measured: tiles with little tensor work per slot -- 1x1 filters on up to 256 channels -- gain nothing: their
-    // time goes to the per-slot hand-offs, and the atomic stores of the cut tiles cost more than the idle SMs did)
-    const bool heavy_slots = p.KHW * CW >= 16 || a.total_tiles < sms;
-    if (allow_balanced && heavy_slots && rows_ok && gate >= 0 && a.total_tiles % sms != 0) {
-        // short layers: as many CTAs as leaves each about four slots to amortise its prologue
-        long long ctas = units / 4;
-        if (ctas < 1) ctas = 1;
-        if (ctas > sms) ctas = sms;
-        const long long waves = (a.total_tiles + sms - 1) / sms;
-        // worth a clearing launch when the last wave of whole tiles would waste more than 1 % of the SM time
-        if ((double)a.total_tiles / sms < 0.99 * (double)waves || ctas > (long long)grid) {
-            a.balanced = 1;
-            grid = (unsigned)ctas;
-        }
+    const TcSplit split = tc_split(p, d, d_pos, d_neg, gate, sms, a.total_tiles);
+    const unsigned grid = split.grid;
+    a.balanced = split.balanced;
+    if (a.balanced == 2 && !outputs_cleared) {
+        const size_t out_bytes = (size_t)p.M * p.Co * sizeof(int16_t);
+        REXSC_CUDA_CHECK(cudaMemsetAsync(d_pos, 0, out_bytes, st));
+        REXSC_CUDA_CHECK(cudaMemsetAsync(d_neg, 0, out_bytes, st));
     }
-    // Outputs without such rows (NCHW, a ragged last chunk): clear them whole and let every tile add single 16-bit
-    // values -- affordable while the outputs are small, which is where whole tiles waste most (deep layers with few
-    // tiles per SM).  The element count must be even so that the last value's 32-bit word ends inside the tensor.
-    const size_t out_elems = (size_t)p.M * p.Co;
-    if (allow_balanced && heavy_slots && !rows_ok && aligned4 && (out_elems & 1) == 0 && out_elems * sizeof(int16_t) <= ((size_t)16 << 20) &&
-        gate >= 0 && a.total_tiles % sms != 0) {
-        long long ctas = units / 4;
-        if (ctas < 1) ctas = 1;
-        if (ctas > sms) ctas = sms;
-        const long long waves = (a.total_tiles + sms - 1) / sms;
-        if ((double)a.total_tiles / sms < 0.95 * (double)waves || ctas > (long long)grid) {
-            a.balanced = 2;
-            grid = (unsigned)ctas;
-            REXSC_CUDA_CHECK(cudaMemsetAsync(d_pos, 0, out_elems * sizeof(int16_t), st));
-            REXSC_CUDA_CHECK(cudaMemsetAsync(d_neg, 0, out_elems * sizeof(int16_t), st));
-        }
-    }
-    if (a.balanced == 1 && grid > 1) {
+    if (a.balanced == 1 && grid > 1 && !outputs_cleared) {
         zero_shared_tiles_kernel<<<grid - 1, kTcM, 0, st>>>(a, (int)grid, d_pos, d_neg, d_status, gate);
         REXSC_LAUNCH_CHECK("zero_shared_tiles_kernel");
     }

@@ -1168,6 +1168,8 @@ struct ExpandAllArgs {
     int gate;          // run only if status[1] != 0
     int verify_vec;    // the border check may use 16-byte loads and 32-bit indices
     int w_vec;         // fp32 weights, input channels fastest, whole 16-byte groups
+    uint4 *clear[2];   // ExpandAllOptions::clear
+    long long clear_n;
     int cw_parts;      // the channel words of a pixel group are shared out to this many warps
 };
 
@@ -1190,6 +1192,10 @@ expand_all_kernel(ExpandAllArgs g, const T *__restrict__ x, const void *__restri
     if (g.gate && status[1] == 0) return; // fallback launch: the compact planes were valid, nothing to redo
     // the device status block of the workspace (when borders are verified the caller has cleared it: word 1 is being set)
     if (!g.verify_border && !g.gate && blockIdx.x == 0 && threadIdx.x < 64) status[threadIdx.x] = 0;
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < g.clear_n; i += (long long)gridDim.x * blockDim.x) {
+        g.clear[0][i] = make_uint4(0u, 0u, 0u, 0u);
+        g.clear[1][i] = make_uint4(0u, 0u, 0u, 0u);
+    }
     if (g.verify_border) {
         // Every border pixel of the padded tensor (rows 0 and Hp-1, columns 0 and Wp-1) must quantise to zero, i.e. be
         // <= 0 (or NaN): the compact grid shares one zero row / column between neighbouring rows / images.
@@ -1432,6 +1438,8 @@ int launch_expand_all_bits(const ConvPlan &p, const rexsc_sc_conv_desc &d, const
     if (opt.skip_weights) g.w_items = 0;
     g.verify_border = opt.verify_border ? 1 : 0;
     g.gate = opt.gate ? 1 : 0;
+    for (int i = 0; i < 2; i++) g.clear[i] = static_cast<uint4 *>(opt.clear[i]);
+    g.clear_n = opt.clear_n;
     g.verify_vec = (!nchw && (long long)p.N * (2LL * p.Wp + 2LL * p.Hp) * p.C < (1LL << 31)) ? 1 : 0;
     const int CW = w.CW;
 #define REXSC_ALL(T) (p.words == 1 ? launch_expand_all_t<T, 1, false>(g, d_act, d_w, d_Ab, d_Wb, d_status, CW, lut_bytes, st)   \
