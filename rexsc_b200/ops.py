@@ -7,7 +7,9 @@ only; all arithmetic happens in librexsc_b200.so.  There is no CPU path: tensors
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes as C
+import functools
 import os
 import threading
 from typing import List, Sequence, Tuple
@@ -17,6 +19,8 @@ import torch
 from . import _lib
 
 _DTYPES = {torch.float32: _lib.F32, torch.float16: _lib.F16, torch.bfloat16: _lib.BF16}
+_raw_stream = torch._C._cuda_getCurrentRawStream if hasattr(torch._C, "_cuda_getCurrentRawStream") else (
+    lambda index: torch.cuda.current_stream(index).cuda_stream)
 _DEBUG = os.environ.get("REXSC_B200_DEBUG", "0") == "1"
 _NVTX = os.environ.get("REXSC_B200_NVTX", "0") == "1"
 
@@ -61,7 +65,7 @@ _workspaces: dict = {}
 
 
 def _workspace(device: torch.device, nbytes: int) -> torch.Tensor:
-    key = (device.index, torch.cuda.current_stream(device).cuda_stream)
+    key = (device.index, _raw_stream(device.index))
     buf = _workspaces.get(key)
     if buf is None or buf.numel() < nbytes:
         buf = torch.empty(max(nbytes, 1 << 20), dtype=torch.uint8, device=device)
@@ -74,12 +78,21 @@ def release_workspaces() -> None:
     _workspaces.clear()
 
 
-def _stream(device) -> C.c_void_p:
-    return C.c_void_p(torch.cuda.current_stream(device).cuda_stream)
+# (the arguments are declared as pointers: plain integers convert without an object of their own)
+def _stream(device) -> int:
+    return _raw_stream(torch.cuda.current_device() if device.index is None else device.index)
 
 
-def _ptr(t: torch.Tensor) -> C.c_void_p:
-    return C.c_void_p(t.data_ptr())
+def _ptr(t: torch.Tensor) -> int:
+    return t.data_ptr()
+
+
+_HERE = contextlib.nullcontext()
+
+
+def _on(device: torch.device):
+    """``torch.cuda.device(device)``, or nothing where that device is current already."""
+    return _HERE if torch.cuda.current_device() == device.index else torch.cuda.device(device)
 
 
 def _require_cuda(t: torch.Tensor, what: str) -> None:
@@ -111,6 +124,32 @@ def _flat_dense(t: torch.Tensor) -> torch.Tensor:
 
 
 # ---- SC conv2d / linear -------------------------------------------------------------------------------
+@functools.lru_cache(maxsize=512)
+def _conv_plan(x_shape, w_shape, x_dtype, w_dtype, a_cl, w_cl, bit_length, lfsr_length, pad_w, pad_h, stride_h, stride_w,
+               prog_total_width, prog_load_width, prog_load_wait, bin_config, gen_config, xnor, kernel):
+    """Descriptor (never written to again), workspace bytes and output size of a conv call: filling the 24 fields and
+    asking for the size cost the host more than its launches, and a program repeats a handful of calls."""
+    d = _lib.ScConvDesc()
+    d.batch, d.c_in, d.h_in, d.w_in = x_shape
+    d.c_out, _, d.kh, d.kw = w_shape
+    d.pad_w, d.pad_h = pad_w, pad_h  # padding[0] pads the last dim (sc_cuda.cpp:88)
+    d.stride_h, d.stride_w = stride_h, stride_w
+    d.act_dtype, d.act_channels_last = _DTYPES[x_dtype], int(a_cl)
+    d.w_dtype, d.w_channels_last = _DTYPES[w_dtype], int(w_cl)
+    d.out_channels_last = int(a_cl)
+    d.bit_length, d.lfsr_length = bit_length, lfsr_length
+    d.bin_config, d.gen_config, d.xnor = bin_config, gen_config, int(xnor)
+    d.prog_total_width, d.prog_load_width, d.prog_load_wait = prog_total_width, prog_load_width, prog_load_wait
+    d.linear_seeds = 0
+    d.kernel = kernel
+    nbytes = _lib.load().rexsc_sc_conv2d_workspace_size(C.byref(d))
+    if nbytes == 0:
+        raise ValueError("conv2d_generic_general_split_acc: unsupported shape or configuration")
+    oh = (d.h_in + 2 * d.pad_h - d.kh) // d.stride_h + 1
+    ow = (d.w_in + 2 * d.pad_w - d.kw) // d.stride_w + 1
+    return d, nbytes, oh, ow
+
+
 @_traced
 def conv2d_generic_general_split_acc(input: torch.Tensor, weight: torch.Tensor, bit_length: int, lfsr_length: int,
                                      z_units: int, padding: Sequence[int], stride: Sequence[int],
@@ -125,29 +164,15 @@ def conv2d_generic_general_split_acc(input: torch.Tensor, weight: torch.Tensor, 
         raise ValueError("conv2d_generic_general_split_acc: expected input [N,C,H,W] and weight [Co,C,KH,KW]")
     lib = _lib.load()
     dev = input.device
-    with torch.cuda.device(dev):
+    with _on(dev):
         a_cl = _is_channels_last(input)
         w_cl = _is_channels_last(weight)
         x = _dense(_float_kind(input), a_cl)
         w = _dense(_float_kind(weight), w_cl)
-        d = _lib.ScConvDesc()
-        d.batch, d.c_in, d.h_in, d.w_in = x.shape
-        d.c_out, _, d.kh, d.kw = w.shape
-        d.pad_w, d.pad_h = int(padding[0]), int(padding[1])  # padding[0] pads the last dim (sc_cuda.cpp:88)
-        d.stride_h, d.stride_w = int(stride[0]), int(stride[1])
-        d.act_dtype, d.act_channels_last = _DTYPES[x.dtype], int(a_cl)
-        d.w_dtype, d.w_channels_last = _DTYPES[w.dtype], int(w_cl)
-        d.out_channels_last = int(a_cl)
-        d.bit_length, d.lfsr_length = int(bit_length), int(lfsr_length)
-        d.bin_config, d.gen_config, d.xnor = int(bin_config), int(gen_config), int(bool(xnor))
-        d.prog_total_width, d.prog_load_width, d.prog_load_wait = (int(v) for v in prog_load)
-        d.linear_seeds = 0
-        d.kernel = _kernel()
-        nbytes = lib.rexsc_sc_conv2d_workspace_size(C.byref(d))
-        if nbytes == 0:
-            raise ValueError("conv2d_generic_general_split_acc: unsupported shape or configuration")
-        oh = (d.h_in + 2 * d.pad_h - d.kh) // d.stride_h + 1
-        ow = (d.w_in + 2 * d.pad_w - d.kw) // d.stride_w + 1
+        tw, lw, lwait = (int(v) for v in prog_load)
+        d, nbytes, oh, ow = _conv_plan(tuple(x.shape), tuple(w.shape), x.dtype, w.dtype, a_cl, w_cl, int(bit_length),
+                                       int(lfsr_length), int(padding[0]), int(padding[1]), int(stride[0]), int(stride[1]),
+                                       tw, lw, lwait, int(bin_config), int(gen_config), bool(xnor), _kernel())
         fmt = torch.channels_last if a_cl else torch.contiguous_format
         if out is None:
             pos = torch.empty((d.batch, d.c_out, oh, ow), dtype=torch.int16, device=dev, memory_format=fmt)
@@ -257,7 +282,7 @@ def workspace_status(device=None) -> int:
     buf = _workspaces.get(key)
     if buf is None:
         return 0
-    with torch.cuda.device(dev):
+    with _on(dev):
         return _lib.load().rexsc_workspace_status(_ptr(buf), _stream(dev))
 
 
@@ -275,7 +300,7 @@ def linear_generic_general_acc(input: torch.Tensor, weight: torch.Tensor, prog_l
         raise ValueError("linear_generic_general_acc: expected input [B,C] and weight [Co,C]")
     lib = _lib.load()
     dev = input.device
-    with torch.cuda.device(dev):
+    with _on(dev):
         x = _float_kind(input).contiguous()
         w = _float_kind(weight).contiguous()
         B, Cin = x.shape
@@ -357,7 +382,7 @@ def or_approx_n_forward_acc(input: torch.Tensor, or_n: int) -> torch.Tensor:
     or_n = _check_or_n(or_n, "or_approx_n_forward_acc")
     lib = _lib.load()
     dev = input.device
-    with torch.cuda.device(dev):
+    with _on(dev):
         x = _flat_dense(_float_kind(input))
         out = torch.empty_like(x, dtype=torch.float32)
         _lib.check(lib.rexsc_orn_fwd(_ptr(x), _DTYPES[x.dtype], _ptr(out), x.numel(), or_n, _stream(dev)),
@@ -379,7 +404,7 @@ def or_approx_n_backward_acc(grad_output: torch.Tensor, input: torch.Tensor, or_
     or_n = _check_or_n(or_n, "or_approx_n_backward_acc")
     lib = _lib.load()
     dev = grad_output.device
-    with torch.cuda.device(dev):
+    with _on(dev):
         g = _flat_dense(grad_output)
         x = _match_layout(_float_kind(input), g)
         out = torch.empty_like(g)
@@ -397,7 +422,7 @@ def or_approx_n_forward_bias_std_both_acc(input_pos: torch.Tensor, input_neg: to
     or_n = _check_or_n(or_n, "or_approx_n_forward_bias_std_both_acc")
     lib = _lib.load()
     dev = input_pos.device
-    with torch.cuda.device(dev):
+    with _on(dev):
         p = _flat_dense(_float_kind(input_pos))
         n = _match_layout(_float_kind(input_neg).to(p.dtype), p)
         b = _coef(bias_coef, dev, "or_approx_n_forward_bias_std_both_acc")
@@ -420,7 +445,7 @@ def or_approx_n_backward_bias_std_both_acc(grad_output: torch.Tensor, input_pos:
     or_n = _check_or_n(or_n, "or_approx_n_backward_bias_std_both_acc")
     lib = _lib.load()
     dev = grad_output.device
-    with torch.cuda.device(dev):
+    with _on(dev):
         g = _flat_dense(grad_output)
         p = _match_layout(_float_kind(input_pos), g)
         n = _match_layout(_float_kind(input_neg).to(p.dtype), g)
@@ -441,7 +466,7 @@ def or_approx_n_forward_bias_std_acc(input: torch.Tensor, bias_coef: torch.Tenso
     or_n = _check_or_n(or_n, "or_approx_n_forward_bias_std_acc")
     lib = _lib.load()
     dev = input.device
-    with torch.cuda.device(dev):
+    with _on(dev):
         x = _flat_dense(_float_kind(input))
         b = _coef(bias_coef, dev, "or_approx_n_forward_bias_std_acc")
         s = _coef(std_coef, dev, "or_approx_n_forward_bias_std_acc")
@@ -461,7 +486,7 @@ def or_approx_n_backward_bias_std_acc(grad_output: torch.Tensor, input: torch.Te
     or_n = _check_or_n(or_n, "or_approx_n_backward_bias_std_acc")
     lib = _lib.load()
     dev = grad_output.device
-    with torch.cuda.device(dev):
+    with _on(dev):
         g = _flat_dense(grad_output)
         x = _match_layout(_float_kind(input), g)
         b = _coef(bias_coef, dev, "or_approx_n_backward_bias_std_acc")
@@ -491,7 +516,7 @@ def sc_counts_to_value(result_pos: torch.Tensor, result_neg: torch.Tensor, bit_l
         raise ValueError("sc_counts_to_value: nothing to compute")
     lib = _lib.load()
     dev = result_pos.device
-    with torch.cuda.device(dev):
+    with _on(dev):
         p = _flat_dense(result_pos)
         n = _match_layout(result_neg, p)
         vp = torch.empty_like(p, dtype=dtype) if split else None
@@ -544,7 +569,7 @@ def sc_calib_stats(result_pos: torch.Tensor, result_neg: torch.Tensor, value_pos
     p, n, gp, gn, gdt = _calib_operands(result_pos, result_neg, value_pos, value_neg, "sc_calib_stats")
     lib = _lib.load()
     dev = p.device
-    with torch.cuda.device(dev):
+    with _on(dev):
         stats = torch.empty((CALIB_BINS * 3 + 1,), dtype=torch.float64, device=dev)
         if between is None:
             _lib.check(lib.rexsc_sc_calib_stats(_ptr(p), _ptr(n), _ptr(gp), _ptr(gn), _DTYPES[gdt], int(bit_length),
@@ -625,7 +650,7 @@ def conv2d_saturate_acc(input: torch.Tensor, weight: torch.Tensor, add_config: i
         raise ValueError("conv2d_saturate_acc: expected input [N,C,H,W] and weight [Co,C,KH,KW]")
     lib = _lib.load()
     dev = input.device
-    with torch.cuda.device(dev):
+    with _on(dev):
         # the reference kernel indexes both tensors as dense NCHW (fixed_cuda_kernel.cu:125,179-182)
         x = _float_kind(input).contiguous()
         w = _float_kind(weight).contiguous()
@@ -658,7 +683,7 @@ def build_lfsr_lut(lfsr_length: int, bit_length: int, gen_config: int = 1, xnor:
     if dev.index is None:
         dev = torch.device("cuda", torch.cuda.current_device())
     words = (bit_length * gen_config + 31) // 32
-    with torch.cuda.device(dev):
+    with _on(dev):
         out = torch.zeros(((1 << lfsr_length) - 1, 1 << lfsr_length, words), dtype=torch.int32, device=dev)
         _lib.check(lib.rexsc_build_lfsr_lut(int(lfsr_length), int(bit_length), int(gen_config), int(bool(xnor)),
                                             int(prog_load[0]), int(prog_load[1]), int(prog_load[2]),
@@ -672,7 +697,7 @@ def alu_probe(blocks: int, iters: int, device="cuda") -> torch.Tensor:
     dev = torch.device(device)
     if dev.index is None:
         dev = torch.device("cuda", torch.cuda.current_device())
-    with torch.cuda.device(dev):
+    with _on(dev):
         sink = torch.empty(blocks * 256, dtype=torch.int32, device=dev)
         _lib.check(lib.rexsc_alu_probe(int(blocks), int(iters), _ptr(sink), _stream(dev)), "rexsc_alu_probe")
     return sink
@@ -684,7 +709,7 @@ def mma_probe(blocks: int, iters: int, n_cols: int = 128, device="cuda") -> torc
     dev = torch.device(device)
     if dev.index is None:
         dev = torch.device("cuda", torch.cuda.current_device())
-    with torch.cuda.device(dev):
+    with _on(dev):
         sink = torch.empty(blocks * 128, dtype=torch.int32, device=dev)
         _lib.check(lib.rexsc_mma_probe(int(blocks), int(iters), int(n_cols), _ptr(sink), _stream(dev)), "rexsc_mma_probe")
     return sink
