@@ -10,13 +10,21 @@
 // output pixels (TMEM lanes) x up to 256 columns.  The products are ordered (tap, channel) with the channels padded
 // to a multiple of 16 -- the order does not matter to the closed form -- and the int8 activations are kept pixel-major
 // (NHWC, same channel padding), so 16 consecutive k' of an output pixel are 16 consecutive bytes in memory.
+//   * k' is taken in slabs of 128 products; a pipeline step is a slab's values and, from the same registers, its
+//     parity bits, so every activation is fetched once and a slab costs one hand-over to the tensor core;
 //   * producers (all 128 threads): fetch the int8 activation slab (128 rows x 128 bytes of k') as eight 16-byte
-//     loads per row through a chunk -> tensor-offset table, and copy the prepacked weight slab, both written to
-//     shared memory in the 128-byte swizzled K-major layout the MMA's shared-memory descriptors name;
-//   * one thread issues tcgen05.mma.kind::i8 (M=128, N=N', K=32) four times per slab and commits to an mbarrier;
+//     loads per row through a chunk -> tensor-offset table, one step ahead (the table's entries two), and the prepacked
+//     weight slabs with asynchronous copies into the other of two buffers, both in the 128-byte swizzled K-major layout
+//     the MMA's shared-memory descriptors name;
+//   * one thread issues tcgen05.mma.kind::i8 (M=128, N=N', K=32) eight times per step and commits to an mbarrier;
 //   * epilogue: tcgen05.ld 32 lanes x 32 columns per warp, min(., cap), pos - neg, coalesced NCHW int32 stores.
+// What bounds it: the latency of a step's gather, hand-over and MMAs, hidden by the other CTAs of the SM where there are
+// enough.  TinyConv's four layers at batch 256, whole calls: 246 us with values and parity bits as separate slabs (every
+// activation fetched twice, table entry and activation one after the other, weights through registers) and three
+// launches, 166 us as it is.
 // Every mbarrier wait is bounded; on a time-out the CTA records it, frees its TMEM and returns.
 #include "common.cuh"
+#include <type_traits>
 
 namespace rexsc {
 
@@ -32,7 +40,7 @@ struct UmmaArgs {
     int H, W, ph, pw; // unpadded activation and the op's zero padding (operand preparation)
     float scale;      // 2^precision_in
     int Cp;          // channels padded to 16 (pixel pitch of the int8 activations, channel pitch of k')
-    int Kp;          // k' extent padded to kSlabBytes (values + parity)
+    int Kp;          // k' extent: per slab of products kSlabBytes of values, then kSlabBytes of parity bits
     int CB, CBp;     // output channels per CTA chunk, padded to 8
     int CBq;         // first MMA column of the negative-weight block (CBp rounded up to 32: aligned TMEM reads)
     int NP;          // MMA N: positive block [0, CBp), negative block [CBq, CBq + CBp), padded to 16
@@ -86,19 +94,18 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity)
     return false;
 }
 
-// PREFETCH_B: also fetch the weight slab one step ahead (64 more registers: two CTAs per SM instead of four) -- pays
-// on grids of at most a wave or two of CTAs, whose time is one CTA's chain of slabs
-template <bool SWIZZLED, bool PREFETCH_B>
-__global__ void __launch_bounds__(128, PREFETCH_B ? 2 : 6)
+template <bool SWIZZLED>
+__global__ void __launch_bounds__(128, 4)
 fxp_conv_umma_kernel(UmmaArgs a, const int8_t *__restrict__ act, const int8_t *__restrict__ wpk,
                      const int32_t *__restrict__ koff, int32_t *__restrict__ out, int *__restrict__ status)
 {
     extern __shared__ __align__(16) uint8_t smem_raw[];
     // the swizzled operand tiles must start on a 1024-byte boundary of the shared window
     uint8_t *smem = smem_raw + ((1024u - (smem_addr(smem_raw) & 1023u)) & 1023u);
-    uint8_t *a_s = smem;                                   // 128 rows x 128 B
-    uint8_t *b_s = smem + kUmmaM * kSlabBytes;             // NP rows x 128 B (1024-byte aligned: 16 KB offset)
-    uint64_t *bar = reinterpret_cast<uint64_t *>(b_s + a.NP * kSlabBytes);        // (the launch sizes the tile by NP)
+    const uint32_t a_tile = kUmmaM * kSlabBytes, b_tile = (uint32_t)((a.NP + 7) / 8 * 8) * kSlabBytes; // 1024-byte multiples
+    uint8_t *a_s = smem;                                   // values, parity bits: 128 rows x 128 B each
+    uint8_t *b_s = smem + 2 * a_tile;                      // [buffer][values, parity bits]: NP rows x 128 B each
+    uint64_t *bar = reinterpret_cast<uint64_t *>(b_s + 4 * b_tile);
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bar + 1);
 
     const int tid = threadIdx.x, warp = tid >> 5;
@@ -132,87 +139,91 @@ fxp_conv_umma_kernel(UmmaArgs a, const int8_t *__restrict__ act, const int8_t *_
     // instruction descriptor: int32 accumulate, signed int8 A and B, both K-major, N = NP, M = 128
     const uint32_t idesc = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(a.NP >> 3) << 17) | ((uint32_t)(kUmmaM >> 4) << 24);
     const int8_t *wchunk = wpk + (size_t)chunk * a.NP * a.Kp;
-    const int n_slabs = a.Kp / kSlabBytes;
+    const int n_steps = a.Kp / (2 * kSlabBytes);
     bool failed = false;
 
-    // The activation words of a slab are fetched into registers one slab ahead: the loads of slab s + 1 are in flight
-    // while the tensor core works through slab s (the shared-memory tiles are single: they are rewritten once those
-    // MMAs are done).  Row = this thread's output pixel, 8 chunks of 16 k' each = 16 channels of one tap.  Weight
-    // slab: NP rows x 8 chunks of the prepacked weights, chunk i * 128 + tid for i < 16 (NP <= 256).
-    uint4 av[8], bv[PREFETCH_B ? 16 : 1];
-    auto load_slab = [&](int slab) {
+    // Row = this thread's output pixel, 8 chunks of 16 products each = 16 channels of one tap.  The chunks of step s + 1
+    // are in flight while the tensor core works through step s, and so are its weight slabs; the table entries they are
+    // fetched through are read another step earlier.
+    uint4 av[8];
+    int off[8];
+    auto load_off = [&](int step) {
+#pragma unroll
+        for (int c = 0; c < 8; c++) off[c] = step < n_steps ? __ldg(koff + step * 8 + c) : -1; // < 0: padding
+    };
+    auto load_act = [&]() {
 #pragma unroll
         for (int c = 0; c < 8; c++) {
             av[c] = make_uint4(0u, 0u, 0u, 0u);
-            const int off = __ldg(koff + slab * 8 + c);         // < 0: padding; bit 30 set: parity operand
-            if (row_live && off >= 0) {
-                av[c] = __ldg(reinterpret_cast<const uint4 *>(act + abase + (off & 0x3fffffff)));
-                if (off & 0x40000000) {
-                    av[c].x &= 0x01010101u; av[c].y &= 0x01010101u; av[c].z &= 0x01010101u; av[c].w &= 0x01010101u;
-                }
-            }
-        }
-        if (PREFETCH_B) {
-#pragma unroll
-            for (int i = 0; i < (PREFETCH_B ? 16 : 1); i++) {
-                const int e = i * 128 + tid, r = e >> 3, c = e & 7;
-                if (e < a.NP * 8)
-                    bv[i] = __ldg(reinterpret_cast<const uint4 *>(wchunk + (size_t)r * a.Kp + slab * kSlabBytes) + c);
-            }
+            if (row_live && off[c] >= 0) av[c] = __ldg(reinterpret_cast<const uint4 *>(act + abase + off[c]));
         }
     };
-    load_slab(0);
-    for (int slab = 0; slab < n_slabs; slab++) {
-#pragma unroll
-        for (int c = 0; c < 8; c++)
-            *reinterpret_cast<uint4 *>(a_s + (SWIZZLED ? sw128_offset(tid, c) : interleaved_offset(tid, c, kUmmaM))) = av[c];
-        if (PREFETCH_B) {
-#pragma unroll
-            for (int i = 0; i < (PREFETCH_B ? 16 : 1); i++) {
-                const int e = i * 128 + tid, r = e >> 3, c = e & 7;
-                if (e < a.NP * 8)
-                    *reinterpret_cast<uint4 *>(b_s + (SWIZZLED ? sw128_offset(r, c) : interleaved_offset(r, c, a.NP))) = bv[i];
-            }
+    auto load_weights = [&](int step) { // NP rows x 16 chunks of 16 bytes (values, then parity bits) -> buffer step & 1
+        const uint32_t dst0 = smem_addr(b_s) + (uint32_t)(step & 1) * 2 * b_tile;
+        for (int e = tid; e < a.NP * 16; e += 128) {
+            const int r = e >> 4, c = e & 7, half = (e >> 3) & 1;
+            const uint32_t dst = dst0 + (uint32_t)half * b_tile + (SWIZZLED ? sw128_offset(r, c) : interleaved_offset(r, c, a.NP));
+            const int8_t *src = wchunk + (size_t)r * a.Kp + (size_t)step * 2 * kSlabBytes + (e & 15) * 16;
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
         }
-        // B slab without prefetch: NP rows x 8 chunks, straight copy of the prepacked weights (L2-resident)
-        for (int i = tid; !PREFETCH_B && i < a.NP * 8; i += blockDim.x) {
-            const int r = i >> 3, c = i & 7;
-            const uint4 v = __ldg(reinterpret_cast<const uint4 *>(wchunk + (size_t)r * a.Kp + slab * kSlabBytes) + c);
-            *reinterpret_cast<uint4 *>(b_s + (SWIZZLED ? sw128_offset(r, c) : interleaved_offset(r, c, a.NP))) = v;
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    load_weights(0);
+    load_off(0);
+    load_act();
+    load_off(1);
+    for (int step = 0; step < n_steps; step++) {
+#pragma unroll
+        for (int c = 0; c < 8; c++) {
+            uint8_t *dst = a_s + (SWIZZLED ? sw128_offset(tid, c) : interleaved_offset(tid, c, kUmmaM));
+            *reinterpret_cast<uint4 *>(dst) = av[c];
+            *reinterpret_cast<uint4 *>(dst + a_tile) =
+                make_uint4(av[c].x & 0x01010101u, av[c].y & 0x01010101u, av[c].z & 0x01010101u, av[c].w & 0x01010101u);
         }
+        asm volatile("cp.async.wait_all;" ::: "memory");
         // generic-proxy writes must be visible to the tensor core's async-proxy reads
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncthreads();
         if (tid == 0) {
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint64_t da = SWIZZLED ? umma_desc_k_sw128(smem_addr(a_s)) : umma_desc_k_interleaved(smem_addr(a_s), kUmmaM);
-            const uint64_t db = SWIZZLED ? umma_desc_k_sw128(smem_addr(b_s)) : umma_desc_k_interleaved(smem_addr(b_s), a.NP);
 #pragma unroll
-            for (int kk = 0; kk < kSlabBytes / kUmmaK; kk++) {
-                const uint32_t accumulate = (slab > 0 || kk > 0) ? 1u : 0u;
-                // advancing K by 32 bytes: +2 address units (16 B) inside a swizzle row, or two K-columns further
-                // in the interleaved layout
-                const uint64_t dak = da + (uint64_t)(SWIZZLED ? kk * (kUmmaK >> 4) : kk * 2 * (kUmmaM * 16 >> 4));
-                const uint64_t dbk = db + (uint64_t)(SWIZZLED ? kk * (kUmmaK >> 4) : kk * 2 * (a.NP * 16 >> 4));
-                asm volatile(
-                    "{\n\t.reg .pred p;\n\t"
-                    "setp.ne.b32 p, %4, 0;\n\t"
-                    "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}"
-                    ::"r"(tmem_base), "l"(dak), "l"(dbk), "r"(idesc), "r"(accumulate), "r"(0u)
-                    : "memory");
+            for (int half = 0; half < 2; half++) { // values, parity bits
+                const uint32_t aa = smem_addr(a_s) + (uint32_t)half * a_tile;
+                const uint32_t bb = smem_addr(b_s) + (uint32_t)((step & 1) * 2 + half) * b_tile;
+                const uint64_t da = SWIZZLED ? umma_desc_k_sw128(aa) : umma_desc_k_interleaved(aa, kUmmaM);
+                const uint64_t db = SWIZZLED ? umma_desc_k_sw128(bb) : umma_desc_k_interleaved(bb, a.NP);
+#pragma unroll
+                for (int kk = 0; kk < kSlabBytes / kUmmaK; kk++) {
+                    const uint32_t accumulate = (step > 0 || half > 0 || kk > 0) ? 1u : 0u;
+                    // advancing K by 32 bytes: +2 address units (16 B) inside a swizzle row, or two K-columns further
+                    // in the interleaved layout
+                    const uint64_t dak = da + (uint64_t)(SWIZZLED ? kk * (kUmmaK >> 4) : kk * 2 * (kUmmaM * 16 >> 4));
+                    const uint64_t dbk = db + (uint64_t)(SWIZZLED ? kk * (kUmmaK >> 4) : kk * 2 * (a.NP * 16 >> 4));
+                    asm volatile(
+                        "{\n\t.reg .pred p;\n\t"
+                        "setp.ne.b32 p, %4, 0;\n\t"
+                        "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}"
+                        ::"r"(tmem_base), "l"(dak), "l"(dbk), "r"(idesc), "r"(accumulate), "r"(0u)
+                        : "memory");
+                }
             }
             asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
                              smem_addr(bar))
                          : "memory");
         }
-        if (slab + 1 < n_slabs) load_slab(slab + 1);
-        // the slab buffers are reused next step: wait until the MMAs that read them have completed
-        if (!mbar_wait(smem_addr(bar), (uint32_t)(slab & 1))) failed = true;
+        if (step + 1 < n_steps) {
+            load_weights(step + 1); // (the MMAs of step - 1, which read that buffer, have completed)
+            load_act();
+            load_off(step + 2);
+        }
+        // the activation tiles are rewritten next step: wait until the MMAs that read them have completed
+        if (!mbar_wait(smem_addr(bar), (uint32_t)(step & 1))) failed = true;
         failed = __syncthreads_or(failed ? 1 : 0) != 0;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         if (failed) break;
     }
+    asm volatile("cp.async.wait_all;" ::: "memory");
 
     if (!failed) {
         // ---- epilogue: this warp reads its 32 TMEM lanes, 32 columns at a time ---------------------------------
@@ -270,47 +281,46 @@ fxp_conv_umma_kernel(UmmaArgs a, const int8_t *__restrict__ act, const int8_t *_
 }
 
 // ---- operand preparation ------------------------------------------------------------------------------------
-// Both kernels quantise on the fly (round-half-even of value * 2^p, fixed_cuda.cpp:28-30: activations clamped to
-// [0, 2^p - 1], weights split into a positive and a negative magnitude), so the tensor-core path needs two launches
-// before the conv kernel instead of four.
-// k' = tap * Cp + c for the values, K2 + tap * Cp + c for the parity bits (K2 = KH * KW * Cp); weights are [co][c][tap]
+// One launch quantises on the fly (round-half-even of value * 2^p, fixed_cuda.cpp:28-30: activations clamped to
+// [0, 2^p - 1], weights split into a positive and a negative magnitude): the first act_blocks blocks write the
+// activations, the others the packed weights and the offset table.
+// k' = slab by slab of 128 products tap * Cp + c: their values, then their parity bits; weights are [co][c][tap]
 template <typename T>
-__global__ void fxp_umma_pack_kernel(UmmaArgs a, int KH, int KW, int n_chunks, const T *__restrict__ w,
-                                     int8_t *__restrict__ wpk, int32_t *__restrict__ koff)
+__device__ __forceinline__ void pack_weights(const UmmaArgs &a, int KH, int KW, int n_chunks, const T *__restrict__ w,
+                                             int8_t *__restrict__ wpk, int32_t *__restrict__ koff, int block, int blocks)
 {
     const int KHW = KH * KW, K2 = KHW * a.Cp;
     // weights: wpk[chunk][row n' in 0..NP)[k' in 0..Kp), row = sign * CBq + local channel
     const long long total = (long long)n_chunks * a.NP * a.Kp;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
-         i += (long long)gridDim.x * blockDim.x) {
+    for (long long i = (long long)block * blockDim.x + threadIdx.x; i < total; i += (long long)blocks * blockDim.x) {
         const int kp = (int)(i % a.Kp);
         const long long r = i / a.Kp;
         const int row = (int)(r % a.NP);
         const int chunk = (int)(r / a.NP);
         const int sign = row >= a.CBq ? 1 : 0, cl = row - sign * a.CBq;
         const int co = chunk * a.CB + cl;
+        const int slab = kp / (2 * kSlabBytes), in = kp - slab * 2 * kSlabBytes;
+        const bool parity = in >= kSlabBytes;
+        const int k = slab * kSlabBytes + (parity ? in - kSlabBytes : in);
         int v = 0;
-        if (cl < a.CB && co < a.Co && kp < 2 * K2) {
-            const int k = kp < K2 ? kp : kp - K2;
+        if (cl < a.CB && co < a.Co && k < K2) {
             const int tap = k / a.Cp, c = k - tap * a.Cp;
             if (c < a.C) {
                 const float x = load_as_float<T>(w, ((long long)co * a.C + c) * KHW + tap) * a.scale;
                 v = sign ? (int)rintf(-fminf(fmaxf(x, 1.f - a.scale), 0.f)) : (int)rintf(fminf(fmaxf(x, 0.f), a.scale - 1.f));
-                if (kp >= K2) v &= 1;
+                if (parity) v &= 1;
             }
         }
         wpk[i] = (int8_t)v;
     }
-    // 16-byte chunk of k' -> byte offset of its 16 channels inside the int8 activations, relative to tap (0,0) of the
-    // output pixel
-    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < a.Kp / 16; j += gridDim.x * blockDim.x) {
-        const int kp = j * 16;
+    // 16-byte chunk of products -> byte offset of its 16 channels inside the int8 activations, relative to tap (0,0) of
+    // the output pixel
+    for (int j = block * blockDim.x + threadIdx.x; j < a.Kp / 32; j += blocks * blockDim.x) {
+        const int k = j * 16;
         int off = -1;
-        if (kp < 2 * K2) {
-            const int k = kp < K2 ? kp : kp - K2;
+        if (k < K2) {
             const int tap = k / a.Cp, cg = k - tap * a.Cp, kh = tap / KW, kw = tap - kh * KW;
             off = (kh * a.Wp + kw) * a.Cp + cg;
-            if (kp >= K2) off |= 0x40000000;
         }
         koff[j] = off;
     }
@@ -318,13 +328,20 @@ __global__ void fxp_umma_pack_kernel(UmmaArgs a, int KH, int KW, int n_chunks, c
 
 // dense NCHW activations -> zero-padded int8 NHWC with the channels padded to Cp; one thread per padded pixel and 16
 // channels
-template <typename T>
-__global__ void fxp_umma_act_kernel(UmmaArgs a, const T *__restrict__ x, int8_t *__restrict__ q8)
+template <typename TA, typename TW>
+__global__ void __launch_bounds__(256) fxp_umma_prep_kernel(UmmaArgs a, int KH, int KW, int n_chunks, int act_blocks,
+                                                            const TA *__restrict__ x, const TW *__restrict__ w,
+                                                            int8_t *__restrict__ q8, int8_t *__restrict__ wpk,
+                                                            int32_t *__restrict__ koff)
 {
+    if ((int)blockIdx.x >= act_blocks) {
+        pack_weights<TW>(a, KH, KW, n_chunks, w, wpk, koff, (int)blockIdx.x - act_blocks, (int)gridDim.x - act_blocks);
+        return;
+    }
     const int groups = a.Cp / 16;
     const long long plane = (long long)a.Hp * a.Wp, total = (long long)a.N * plane * groups;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
-         i += (long long)gridDim.x * blockDim.x) {
+         i += (long long)act_blocks * blockDim.x) {
         // consecutive threads take consecutive pixels of one channel group: the strided reads coalesce
         const long long pix = i % plane;
         const long long t = i / plane;
@@ -337,7 +354,7 @@ __global__ void fxp_umma_act_kernel(UmmaArgs a, const T *__restrict__ x, int8_t 
             for (int b = 0; b < 16; b++) {
                 const int c = g * 16 + b;
                 if (c < a.C) {
-                    const float v = load_as_float<T>(x, (((long long)n * a.C + c) * a.H + hi) * a.W + wi) * a.scale;
+                    const float v = load_as_float<TA>(x, (((long long)n * a.C + c) * a.H + hi) * a.W + wi) * a.scale;
                     const int q = (int)rintf(fminf(fmaxf(v, 0.f), a.scale - 1.f));
                     w[b >> 2] |= (uint32_t)(q & 0xff) << (8 * (b & 3));
                 }
@@ -360,7 +377,7 @@ size_t fxp_umma_workspace_bytes(int N, int C, int Hp, int Wp, int Co, long long 
     const int CB = Co < 128 ? Co : 128;
     const int n_chunks = (Co + CB - 1) / CB;
     const int Cp = (C + 15) / 16 * 16;
-    const long long Kp = (2 * umma_k2(C, K) + kSlabBytes - 1) / kSlabBytes * kSlabBytes;
+    const long long Kp = 2 * ((umma_k2(C, K) + kSlabBytes - 1) / kSlabBytes * kSlabBytes);
     return align_up((size_t)N * Hp * Wp * Cp, 256) + align_up((size_t)n_chunks * 256 * Kp, 256) +
            align_up((size_t)Kp * 4, 256);
 }
@@ -381,7 +398,7 @@ int launch_fxp_conv_umma(int N, int C, int H, int W, int ph, int pw, int Co, int
     a.N = N; a.C = C; a.Hp = Hp; a.Wp = Wp; a.Co = Co; a.OH = OH; a.OW = OW; a.sh = sh; a.sw = sw;
     a.H = H; a.W = W; a.ph = ph; a.pw = pw; a.scale = scale;
     a.Cp = (C + 15) / 16 * 16;
-    a.Kp = (int)((2 * umma_k2(C, K) + kSlabBytes - 1) / kSlabBytes * kSlabBytes);
+    a.Kp = (int)(2 * ((umma_k2(C, K) + kSlabBytes - 1) / kSlabBytes * kSlabBytes));
     a.CB = Co < 128 ? Co : 128;
     a.CBp = (a.CB + 7) / 8 * 8;
     a.CBq = (a.CBp + 31) / 32 * 32;
@@ -399,26 +416,30 @@ int launch_fxp_conv_umma(int N, int C, int H, int W, int ph, int pw, int Co, int
                                                 align_up((size_t)n_chunks * a.NP * a.Kp, 256));
     const long long n_act = (long long)N * Hp * Wp * (a.Cp / 16); // one thread per pixel and 16 channels
     const unsigned ab = (unsigned)((n_act + 255) / 256 < 148 * 16 ? (n_act + 255) / 256 : 148 * 16);
+    const long long pack_items = (long long)n_chunks * a.NP * a.Kp;
+    const unsigned pb = (unsigned)((pack_items + 255) / 256 < 148 * 4 ? (pack_items + 255) / 256 : 148 * 4);
+    auto prep = [&](auto *x, auto *w) {
+        using TA = std::remove_const_t<std::remove_pointer_t<decltype(x)>>;
+        using TW = std::remove_const_t<std::remove_pointer_t<decltype(w)>>;
+        fxp_umma_prep_kernel<TA, TW><<<ab + pb, 256, 0, st>>>(a, KH, KW, n_chunks, (int)ab, x, w, q8, wpk, koff);
+    };
+    auto prep_w = [&](auto *x) {
+        switch (w_dtype) {
+        case REXSC_F32: prep(x, (const float *)d_w); break;
+        case REXSC_F16: prep(x, (const __half *)d_w); break;
+        default: prep(x, (const __nv_bfloat16 *)d_w); break;
+        }
+    };
     switch (act_dtype) {
-    case REXSC_F32: fxp_umma_act_kernel<float><<<ab, 256, 0, st>>>(a, (const float *)d_act, q8); break;
-    case REXSC_F16: fxp_umma_act_kernel<__half><<<ab, 256, 0, st>>>(a, (const __half *)d_act, q8); break;
-    default: fxp_umma_act_kernel<__nv_bfloat16><<<ab, 256, 0, st>>>(a, (const __nv_bfloat16 *)d_act, q8); break;
+    case REXSC_F32: prep_w((const float *)d_act); break;
+    case REXSC_F16: prep_w((const __half *)d_act); break;
+    default: prep_w((const __nv_bfloat16 *)d_act); break;
     }
-    REXSC_LAUNCH_CHECK("fxp_umma_act_kernel");
-    switch (w_dtype) {
-    case REXSC_F32: fxp_umma_pack_kernel<float><<<148 * 4, 256, 0, st>>>(a, KH, KW, n_chunks, (const float *)d_w, wpk, koff); break;
-    case REXSC_F16: fxp_umma_pack_kernel<__half><<<148 * 4, 256, 0, st>>>(a, KH, KW, n_chunks, (const __half *)d_w, wpk, koff); break;
-    default:
-        fxp_umma_pack_kernel<__nv_bfloat16><<<148 * 4, 256, 0, st>>>(a, KH, KW, n_chunks, (const __nv_bfloat16 *)d_w, wpk, koff);
-        break;
-    }
-    REXSC_LAUNCH_CHECK("fxp_umma_pack_kernel");
+    REXSC_LAUNCH_CHECK("fxp_umma_prep_kernel");
     // operand tiles sized by the layer: narrow layers fit more CTAs per SM, which is what hides their load latency
-    const size_t smem = (size_t)kUmmaM * kSlabBytes + (size_t)a.NP * kSlabBytes + 64 + 1024;
+    const size_t smem = 2 * (size_t)kUmmaM * kSlabBytes + 4 * (size_t)((a.NP + 7) / 8 * 8) * kSlabBytes + 64 + 1024;
     dim3 grid((unsigned)((a.M + kUmmaM - 1) / kUmmaM), (unsigned)n_chunks);
-    const bool few_ctas = (long long)grid.x * grid.y <= 2 * 148;
-    auto kernel = swizzled ? (few_ctas ? fxp_conv_umma_kernel<true, true> : fxp_conv_umma_kernel<true, false>)
-                           : (few_ctas ? fxp_conv_umma_kernel<false, true> : fxp_conv_umma_kernel<false, false>);
+    auto kernel = swizzled ? fxp_conv_umma_kernel<true> : fxp_conv_umma_kernel<false>;
     REXSC_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     kernel<<<grid, 128, smem, st>>>(a, q8, wpk, koff, out, status);
     REXSC_LAUNCH_CHECK("fxp_conv_umma_kernel");

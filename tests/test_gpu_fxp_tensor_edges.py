@@ -1,0 +1,25 @@
+"""Edges of the tensor-core FXP conv: products that fill a slab of 128 exactly, leave a remainder or need only one;
+pixels around a tile of 128; chunks of 128 output channels.  Integer work: equal to the CUDA-core kernel, which the
+oracle tests cover."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n,c,h,w,co,k,pad", [
+    (1, 1, 1, 1, 1, 1, 0), (1, 16, 8, 16, 8, 1, 0), (2, 128, 8, 8, 16, 1, 0), (1, 129, 8, 16, 33, 1, 0),
+    (3, 3, 11, 13, 32, 5, 2), (1, 8, 9, 9, 130, 4, 0), (2, 17, 10, 7, 64, 3, 1), (5, 64, 4, 4, 10, 4, 0)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+def test_tensor_kernel_equals_cuda_kernel(ops, n, c, h, w, co, k, pad, dtype):
+    g = torch.Generator(device="cuda").manual_seed(c * 100 + co)
+    x = torch.rand(n, c, h, w, device="cuda", generator=g).to(dtype)
+    wt = (torch.randn(co, c, k, k, device="cuda", generator=g) * 0.2).clamp(-1, 1)
+    out = {}
+    for kernel in ("tensor", "tensor_unswizzled", "cuda"):
+        ops.set_fxp_kernel(kernel)
+        try:
+            out[kernel] = ops.conv2d_saturate_acc(x, wt, 0, 5, 24, (pad, pad), (1, 1))
+        finally:
+            ops.set_fxp_kernel("auto")
+    assert torch.equal(out["tensor"], out["cuda"]) and torch.equal(out["tensor_unswizzled"], out["cuda"])
