@@ -20,7 +20,7 @@ One JSON line is printed by rank 0:
              them under autocast; `e2e_fp32_activations` repeats it with fp32 activations); --e2e-slots / --e2e-chunks
              set the staging depth and the batch slicing of the host pipeline
   gpu_launches  this library's kernels inside the timed region, as the library counts them
-  roofline   dominant kernel: the tensor-core SC conv (one int8 tcgen05 GEMM per time slot) against the int8 tensor
+  roofline   dominant kernel: the tensor-core SC conv (one 4-bit tcgen05 GEMM per time slot) against the 4-bit tensor
              rate measured live by a back-to-back MMA probe; `roofline_secondary` / `roofline_expand` the ALU kernel
              and the stream-expansion stage; `roofline_pointwise` the four point-wise kernels against HBM
   train      images/s of full training steps (fwd + bwd + optimizer) of the reference's own model and loop on the
@@ -405,7 +405,7 @@ def run_sc(args, wl, rank, world, local_rank):
         k["ms"] += best["accumulate"] * l["rep"]
         k["products"] += l["rep"] * products
         k["launches"] += l["rep"]
-        k["intops"] += l["rep"] * 4.0 * slots * products          # int8 ops of the per-slot GEMMs
+        k["intops"] += l["rep"] * 4.0 * slots * products          # ops of the per-slot GEMMs
         k["lop3"] += l["rep"] * float(lop3_per_product) * products * ((slots + 31) // 32)
         # DRAM bytes the accumulate kernel has to move: the activation bit planes once + both int16 outputs
         k["bytes"] += l["rep"] * (plane_bytes + 2 * 2 * d.batch * oh * oh * d.c_out)
@@ -471,9 +471,10 @@ def sc_line(args, wl, r, world):
     tc_achieved = t["intops"] / (t["ms"] * 1e-3) if t["ms"] > 0 else 0.0
     alu_achieved = a["lop3"] / (a["ms"] * 1e-3) if a["ms"] > 0 else 0.0
     roof_tensor = {
-        "bound": "tensor", "kernel": "sc_conv_tc_kernel (tcgen05 int8, one GEMM per time slot)",
-        "achieved": tc_achieved / 1e12, "peak": r["mma_peak_ops"] / 1e12, "unit": "TOP/s int8",
-        "frac": tc_achieved / r["mma_peak_ops"],
+        "bound": "tensor", "kernel": "sc_conv_tc_kernel (tcgen05 mxf4, one GEMM per time slot)",
+        # the 4-bit kind takes K = 64 in the clocks that int8 takes K = 32 (both 67 clk for M128 N128): twice the probe rate
+        "achieved": tc_achieved / 1e12, "peak": 2 * r["mma_peak_ops"] / 1e12, "unit": "TOP/s 4-bit",
+        "frac": tc_achieved / (2 * r["mma_peak_ops"]),
         # per average launch: reads = 1.23 x the activation bit planes, the ratio of ncu's dram__bytes_read.sum
         # (65.6 MB) to the planes (53.2 MB) of the captured 64-channel layer at batch 64 (patch halos, the
         # read-modify-write of cut tiles and the weight planes make up the rest; it grows in proportion to the batch);
@@ -505,7 +506,7 @@ def sc_line(args, wl, r, world):
         "metric": wl["metric"], "value": value, "unit": "img/s",
         "n_gpus": world, "steps": args.steps, "warmup": args.warmup, "ms_per_step": r["ms"] / args.steps,
         "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
-        "dtype": "u32 bit-streams / int8 tensor-core operands, int32 accumulators / int16 sums", "data": "synthetic",
+        "dtype": "u32 bit-streams / 0-1 tensor-core operands (e2m1, exact), fp32 integer counts / int16 sums", "data": "synthetic",
         "config": {
             "workload": wl["text"], "batch_per_gpu": batch,
             "parallelism": f"batch-sharded x{world}, no data-path collective on the forward ops "

@@ -43,7 +43,7 @@ enum {
 enum { REXSC_F32 = 0, REXSC_F16 = 1, REXSC_BF16 = 2 };
 
 /* Which SC conv kernel to use; all give identical results.  DIRECT: one thread per output, any shape and any n.
- * TILED: shared-memory implicit GEMM on the integer ALU pipe (LOP3 thermometers).  TENSOR: one int8 tcgen05 GEMM
+ * TILED: shared-memory implicit GEMM on the integer ALU pipe (LOP3 thermometers).  TENSOR: one 4-bit tcgen05 GEMM
  * per time slot with min(count, n) applied to the TMEM accumulators (filters of at most 9 taps, any stride whose
  * residue planes fit its shared-memory patch).  AUTO picks TENSOR whenever the shape fits it and there are at least
  * 32 input channels, else TILED when the shape fits that, else DIRECT. */
@@ -307,8 +307,8 @@ int rexsc_fxp_conv2d_fwd(const rexsc_fxp_conv_desc *desc, const void *d_act, con
 int rexsc_alu_probe(int32_t blocks, int32_t iters, uint32_t *d_sink, void *stream);
 
 /*
- * Tensor-pipe probe used by the benchmark to measure the int8 tcgen05 rate the tensor-core SC conv kernel is measured
- * against: `blocks` CTAs (two fit an SM) each issue iters x 16 int8 MMAs of shape M128 x n_cols x K32 (n_cols 128
+ * Tensor-pipe probe used by the benchmark to measure the int8 tcgen05 rate; the tensor-core SC conv kernel is measured
+ * against twice that, the rate of its 4-bit kind: `blocks` CTAs (two fit an SM) each issue iters x 16 int8 MMAs of shape M128 x n_cols x K32 (n_cols 128
  * or 256) on fixed shared-memory operands.  Total multiply-accumulates = blocks*iters*16*128*n_cols*32.
  * d_sink receives blocks*128 words.
  */
