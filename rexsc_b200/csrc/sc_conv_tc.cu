@@ -36,8 +36,8 @@
 // scales (the same columns serve both operands), 8 of the bias MMA's weights.
 //
 // One persistent CTA per SM walks its tiles as a single pipeline (a tile's first loads and its store overlap the
-// neighbouring tiles' MMAs): eight warps fold counts, four expand operands, one issues the MMAs, unit 0 then unit 1 of
-// every step.  A pipeline step is one slot x one chunk of 64 channels (1x1 filters: up to 256).  Operand buffers are
+// neighbouring tiles' MMAs): 16 warps fold counts, eight expand operands, one copies weight words, one issues the MMAs,
+// unit 0 then unit 1 of every step.  A pipeline step is one slot x one chunk of 64 channels (1x1 filters: up to 256).  Operand buffers are
 // double-buffered, a unit's accumulators are folded while the other unit is computed, and every dependence is an
 // mbarrier phase: while the tensor core works through step i, the folding warps are on the unit that finished and
 // the expanding warps write the operands of step i+1.
