@@ -69,6 +69,11 @@ constexpr int kTcCout = 64;        // output channels per CTA
 constexpr int kTcN = 2 * kTcCout;  // weight rows (MMA M, TMEM lanes): positive block [0,64), negative block [64,128)
 constexpr int kTcMaxTaps = 9;      // filter taps whose weight operand is staged at once
 constexpr int kTcMaxARows = 8;     // patch rows per expanding thread (all residue planes together)
+// Which layers the path takes: residue planes x (256 + tap halo) up to this many rows.  The patch below would hold some
+// more; but a layer on this path needs up to 14 times the workspace of the ALU kernels (bit planes of 32-channel words
+// beside theirs, whichever kernel runs), so taking more layers would put calls that run today beyond the fixed scratch of
+// rexsc_sc_conv2d_fwd_static, or beyond the card (stride 2 on 298 x 298 maps: 71 -> 165 GB at batch 691).
+constexpr int kTcMaxPlaneRows = 1536, kTcPlaneTile = 256;
 constexpr int kTcWordCols = 4;     // TMEM columns of one 32-channel weight word (8 nibbles per column)
 constexpr int kTcMaxWords = 18;    // weight words per row and step: the operand buffers' TMEM columns / kTcWordCols
 constexpr uint32_t kTcColA = 2 * kTcUnit;                                   // first column of the weight buffers
@@ -852,6 +857,8 @@ TcGeom tc_geometry(const ConvPlan &p)
         }
     g.Mh = (kTcM + max_shift + 7) / 8 * 8;
     g.rows_a = g.planes * g.Mh;
+    static_assert((kTcM - kTcPlaneTile) % 8 == 0, "Mh is rounded to 8 rows");
+    if (g.planes * (g.Mh - (kTcM - kTcPlaneTile)) > kTcMaxPlaneRows) return g;
     if (g.rows_a > kTcMaxARows * (kTcExpandWarps * 32)) return g;
     for (int t = 0; t < kTcMaxTaps; t++) g.tap_off[t] = 0;
     for (int kh = 0; kh < p.KH; kh++)

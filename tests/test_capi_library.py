@@ -130,3 +130,30 @@ def test_ops_refuse_cpu_tensors():
         ops.or_approx_n_forward_acc(torch.zeros(4), 2)
     with pytest.raises(RuntimeError):
         ops.conv2d_saturate_acc(torch.zeros(1, 1, 4, 4), torch.zeros(1, 1, 3, 3), 0, 5, 24, (0, 0), (1, 1))
+
+
+# stride 2 / 3 filters whose patch is larger than the tensor-core kernel takes, and the two nearest that it does take
+@pytest.mark.parametrize("shape, tensor", [
+    (dict(batch=4, c_in=64, h_in=30, w_in=30, c_out=64, stride_h=2, stride_w=3), False),   # six residue planes
+    (dict(batch=8, c_in=20, h_in=60, w_in=60, c_out=64, stride_h=3, stride_w=2), False),
+    (dict(batch=1, c_in=32, h_in=24, w_in=260, c_out=64, stride_h=2, stride_w=2), False),  # 4 x (256 + 131) > 1536
+    (dict(batch=1, c_in=32, h_in=24, w_in=252, c_out=64, stride_h=2, stride_w=2), True),   # 4 x (256 + 127 -> 128) = 1536
+    (dict(batch=1, c_in=32, h_in=24, w_in=254, c_out=64, stride_h=2, stride_w=2), True),
+    (dict(batch=1, c_in=32, h_in=24, w_in=256, c_out=64, stride_h=2, stride_w=2), False)])
+def test_layers_on_the_tensor_path(lib, shape, tensor):
+    """Which layers the tensor-core kernel takes, and that the others are not charged for its bit planes: their scratch
+    stays that of the ALU kernels, so a call on the fixed scratch is not refused for planes that it does not use."""
+    from rexsc_b200 import _lib
+
+    forced = _desc(kernel=_lib.KERNEL_TENSOR, **shape)
+    assert lib.rexsc_sc_conv2d_kernel_choice(C.byref(forced)) == (_lib.KERNEL_TENSOR if tensor else -2)
+    auto = _desc(**shape)
+    choice = lib.rexsc_sc_conv2d_kernel_choice(C.byref(auto))
+    assert (choice == _lib.KERNEL_TENSOR) == (tensor and shape["c_in"] >= 32)
+    if not tensor:
+        # stream words of the padded-to-8 channels (row pitch padded by less than 32 words), weights, signs and tables
+        rows = -(-shape["h_in"] // shape["stride_h"]) * min(3, shape["stride_h"])
+        pitch = -(-shape["w_in"] // shape["stride_w"]) * min(3, shape["stride_w"]) + 31
+        c_pad = -(-shape["c_in"] // 8) * 8
+        words = shape["batch"] * rows * pitch * c_pad + 3 * 64 * c_pad * 9
+        assert lib.rexsc_sc_conv2d_workspace_size(C.byref(auto)) <= words * 4 + (1 << 18)
