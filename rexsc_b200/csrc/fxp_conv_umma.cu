@@ -14,14 +14,14 @@
 //     parity bits, so every activation is fetched once and a slab costs one hand-over to the tensor core;
 //   * producers (all 128 threads): fetch the int8 activation slab (128 rows x 128 bytes of k') as eight 16-byte
 //     loads per row through a chunk -> tensor-offset table, one step ahead (the table's entries two), and the prepacked
-//     weight slabs with asynchronous copies into the other of two buffers, both in the 128-byte swizzled K-major layout
-//     the MMA's shared-memory descriptors name;
+//     weight slabs with asynchronous copies (into the other of two buffers where a CTA has its SM to itself), both in the
+//     128-byte swizzled K-major layout the MMA's shared-memory descriptors name;
 //   * one thread issues tcgen05.mma.kind::i8 (M=128, N=N', K=32) eight times per step and commits to an mbarrier;
 //   * epilogue: tcgen05.ld 32 lanes x 32 columns per warp, min(., cap), pos - neg, coalesced NCHW int32 stores.
 // What bounds it: the latency of a step's gather, hand-over and MMAs, hidden by the other CTAs of the SM where there are
 // enough.  TinyConv's four layers at batch 256, whole calls: 246 us with values and parity bits as separate slabs (every
 // activation fetched twice, table entry and activation one after the other, weights through registers) and three
-// launches, 166 us as it is.
+// launches, 155 us as it is.
 // Every mbarrier wait is bounded; on a time-out the CTA records it, frees its TMEM and returns.
 #include "common.cuh"
 #include <type_traits>
@@ -40,11 +40,13 @@ struct UmmaArgs {
     int H, W, ph, pw; // unpadded activation and the op's zero padding (operand preparation)
     float scale;      // 2^precision_in
     int Cp;          // channels padded to 16 (pixel pitch of the int8 activations, channel pitch of k')
+    int K2;          // products: taps x Cp
     int Kp;          // k' extent: per slab of products kSlabBytes of values, then kSlabBytes of parity bits
     int CB, CBp;     // output channels per CTA chunk, padded to 8
     int CBq;         // first MMA column of the negative-weight block (CBp rounded up to 32: aligned TMEM reads)
     int NP;          // MMA N: positive block [0, CBp), negative block [CBq, CBq + CBp), padded to 16
     int tmem_cols;   // power of two >= NP, >= 32
+    int w_bufs;      // buffers of the weight slabs: 2 (those of the next step are copied during a step's MMAs) or 1
     int cap;
     long long M;
 };
@@ -105,7 +107,8 @@ fxp_conv_umma_kernel(UmmaArgs a, const int8_t *__restrict__ act, const int8_t *_
     const uint32_t a_tile = kUmmaM * kSlabBytes, b_tile = (uint32_t)((a.NP + 7) / 8 * 8) * kSlabBytes; // 1024-byte multiples
     uint8_t *a_s = smem;                                   // values, parity bits: 128 rows x 128 B each
     uint8_t *b_s = smem + 2 * a_tile;                      // [buffer][values, parity bits]: NP rows x 128 B each
-    uint64_t *bar = reinterpret_cast<uint64_t *>(b_s + 4 * b_tile);
+    const int n_steps = a.Kp / (2 * kSlabBytes);
+    uint64_t *bar = reinterpret_cast<uint64_t *>(b_s + 2 * a.w_bufs * b_tile);
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bar + 1);
 
     const int tid = threadIdx.x, warp = tid >> 5;
@@ -139,14 +142,18 @@ fxp_conv_umma_kernel(UmmaArgs a, const int8_t *__restrict__ act, const int8_t *_
     // instruction descriptor: int32 accumulate, signed int8 A and B, both K-major, N = NP, M = 128
     const uint32_t idesc = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(a.NP >> 3) << 17) | ((uint32_t)(kUmmaM >> 4) << 24);
     const int8_t *wchunk = wpk + (size_t)chunk * a.NP * a.Kp;
-    const int n_steps = a.Kp / (2 * kSlabBytes);
     bool failed = false;
 
     // Row = this thread's output pixel, 8 chunks of 16 products each = 16 channels of one tap.  The chunks of step s + 1
     // are in flight while the tensor core works through step s, and so are its weight slabs; the table entries they are
     // fetched through are read another step earlier.
+    // Of a last slab only the 32-product blocks that hold products are copied and multiplied (1, 2 or 4 of the 4).
     uint4 av[8];
     int off[8];
+    auto log_blocks = [&](int step) {
+        const int left = a.K2 - step * kSlabBytes;
+        return left <= kUmmaK ? 0 : left <= 2 * kUmmaK ? 1 : 2;
+    };
     auto load_off = [&](int step) {
 #pragma unroll
         for (int c = 0; c < 8; c++) off[c] = step < n_steps ? __ldg(koff + step * 8 + c) : -1; // < 0: padding
@@ -158,12 +165,13 @@ fxp_conv_umma_kernel(UmmaArgs a, const int8_t *__restrict__ act, const int8_t *_
             if (row_live && off[c] >= 0) av[c] = __ldg(reinterpret_cast<const uint4 *>(act + abase + off[c]));
         }
     };
-    auto load_weights = [&](int step) { // NP rows x 16 chunks of 16 bytes (values, then parity bits) -> buffer step & 1
-        const uint32_t dst0 = smem_addr(b_s) + (uint32_t)(step & 1) * 2 * b_tile;
-        for (int e = tid; e < a.NP * 16; e += 128) {
-            const int r = e >> 4, c = e & 7, half = (e >> 3) & 1;
+    auto load_weights = [&](int step) { // NP rows x 2 blocks of 16-byte chunks (values, then parity bits) -> buffer step & 1
+        const uint32_t dst0 = smem_addr(b_s) + (uint32_t)(step & (a.w_bufs - 1)) * 2 * b_tile;
+        const int lc = log_blocks(step) + 1; // log2 of the chunks of a row and half
+        for (int e = tid; e < a.NP << (lc + 1); e += 128) {
+            const int r = e >> (lc + 1), c = e & ((1 << lc) - 1), half = (e >> lc) & 1;
             const uint32_t dst = dst0 + (uint32_t)half * b_tile + (SWIZZLED ? sw128_offset(r, c) : interleaved_offset(r, c, a.NP));
-            const int8_t *src = wchunk + (size_t)r * a.Kp + (size_t)step * 2 * kSlabBytes + (e & 15) * 16;
+            const int8_t *src = wchunk + (size_t)r * a.Kp + (size_t)step * 2 * kSlabBytes + half * kSlabBytes + c * 16;
             asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
@@ -173,8 +181,10 @@ fxp_conv_umma_kernel(UmmaArgs a, const int8_t *__restrict__ act, const int8_t *_
     load_act();
     load_off(1);
     for (int step = 0; step < n_steps; step++) {
+        const int blocks = 1 << log_blocks(step);
 #pragma unroll
         for (int c = 0; c < 8; c++) {
+            if (c >= 2 * blocks) break;
             uint8_t *dst = a_s + (SWIZZLED ? sw128_offset(tid, c) : interleaved_offset(tid, c, kUmmaM));
             *reinterpret_cast<uint4 *>(dst) = av[c];
             *reinterpret_cast<uint4 *>(dst + a_tile) =
@@ -190,11 +200,12 @@ fxp_conv_umma_kernel(UmmaArgs a, const int8_t *__restrict__ act, const int8_t *_
 #pragma unroll
             for (int half = 0; half < 2; half++) { // values, parity bits
                 const uint32_t aa = smem_addr(a_s) + (uint32_t)half * a_tile;
-                const uint32_t bb = smem_addr(b_s) + (uint32_t)((step & 1) * 2 + half) * b_tile;
+                const uint32_t bb = smem_addr(b_s) + (uint32_t)((step & (a.w_bufs - 1)) * 2 + half) * b_tile;
                 const uint64_t da = SWIZZLED ? umma_desc_k_sw128(aa) : umma_desc_k_interleaved(aa, kUmmaM);
                 const uint64_t db = SWIZZLED ? umma_desc_k_sw128(bb) : umma_desc_k_interleaved(bb, a.NP);
 #pragma unroll
                 for (int kk = 0; kk < kSlabBytes / kUmmaK; kk++) {
+                    if (kk >= blocks) break;
                     const uint32_t accumulate = (step > 0 || half > 0 || kk > 0) ? 1u : 0u;
                     // advancing K by 32 bytes: +2 address units (16 B) inside a swizzle row, or two K-columns further
                     // in the interleaved layout
@@ -213,7 +224,7 @@ fxp_conv_umma_kernel(UmmaArgs a, const int8_t *__restrict__ act, const int8_t *_
                          : "memory");
         }
         if (step + 1 < n_steps) {
-            load_weights(step + 1); // (the MMAs of step - 1, which read that buffer, have completed)
+            if (a.w_bufs == 2) load_weights(step + 1); // (the MMAs of step - 1, which read that buffer, have completed)
             load_act();
             load_off(step + 2);
         }
@@ -222,6 +233,7 @@ fxp_conv_umma_kernel(UmmaArgs a, const int8_t *__restrict__ act, const int8_t *_
         failed = __syncthreads_or(failed ? 1 : 0) != 0;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         if (failed) break;
+        if (a.w_bufs == 1 && step + 1 < n_steps) load_weights(step + 1);
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
 
@@ -398,6 +410,7 @@ int launch_fxp_conv_umma(int N, int C, int H, int W, int ph, int pw, int Co, int
     a.N = N; a.C = C; a.Hp = Hp; a.Wp = Wp; a.Co = Co; a.OH = OH; a.OW = OW; a.sh = sh; a.sw = sw;
     a.H = H; a.W = W; a.ph = ph; a.pw = pw; a.scale = scale;
     a.Cp = (C + 15) / 16 * 16;
+    a.K2 = (int)umma_k2(C, K);
     a.Kp = (int)(2 * ((umma_k2(C, K) + kSlabBytes - 1) / kSlabBytes * kSlabBytes));
     a.CB = Co < 128 ? Co : 128;
     a.CBp = (a.CB + 7) / 8 * 8;
@@ -436,8 +449,15 @@ int launch_fxp_conv_umma(int N, int C, int H, int W, int ph, int pw, int Co, int
     default: prep_w((const __nv_bfloat16 *)d_act); break;
     }
     REXSC_LAUNCH_CHECK("fxp_umma_prep_kernel");
-    // operand tiles sized by the layer: narrow layers fit more CTAs per SM, which is what hides their load latency
-    const size_t smem = 2 * (size_t)kUmmaM * kSlabBytes + 4 * (size_t)((a.NP + 7) / 8 * 8) * kSlabBytes + 64 + 1024;
+    // Operand tiles sized by the layer: narrow layers fit more CTAs per SM, which is what hides a step's latency.  So does a
+    // single weight buffer, and where there are more CTAs than SMs it hides more than the copy of the next step's weights
+    // during the MMAs does (whole calls, two buffers -> one): 3x3 17 -> 497 channels, 172 CTAs: 35 -> 27 us; 5x5 33 -> 45,
+    // 1319 CTAs: 123 -> 94 us; TinyConv 165 -> 155 us; with the empty blocks of its only slab left out as well, 1x1 7 -> 83
+    // on 160 x 61 x 61: 228 -> 130 us (171 us with values and parity bits in one slab).  With a CTA per SM
+    // and no other to hide behind the second buffer is the better one: 4x4 134 -> 78 channels, 19 CTAs: 35 against 37 us.
+    const long long ctas = (a.M + kUmmaM - 1) / kUmmaM * n_chunks;
+    a.w_bufs = a.Kp > 2 * kSlabBytes && ctas <= 148 ? 2 : 1;
+    const size_t smem = 2 * (size_t)kUmmaM * kSlabBytes + 2 * a.w_bufs * (size_t)((a.NP + 7) / 8 * 8) * kSlabBytes + 64 + 1024;
     dim3 grid((unsigned)((a.M + kUmmaM - 1) / kUmmaM), (unsigned)n_chunks);
     auto kernel = swizzled ? fxp_conv_umma_kernel<true> : fxp_conv_umma_kernel<false>;
     REXSC_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));

@@ -23,3 +23,22 @@ def test_tensor_kernel_equals_cuda_kernel(ops, n, c, h, w, co, k, pad, dtype):
         finally:
             ops.set_fxp_kernel("auto")
     assert torch.equal(out["tensor"], out["cuda"]) and torch.equal(out["tensor_unswizzled"], out["cuda"])
+
+
+@pytest.mark.parametrize("c,k", [(4, 1), (16, 1), (17, 1), (33, 1), (59, 1), (64, 1), (65, 1), (128, 1), (130, 1), (160, 1),
+                                 (176, 1), (15, 3), (33, 3), (50, 2)])
+@pytest.mark.parametrize("co", [10, 83, 300])
+def test_blocks_of_a_last_slab(ops, c, k, co):
+    """One step and several; last slabs of one, two, three and four blocks of 32 products; one to three channel chunks."""
+    g = torch.Generator(device="cuda").manual_seed(c * 1000 + co)
+    x = torch.rand(3, c, 9, 12, device="cuda", generator=g)
+    wt = (torch.randn(co, c, k, k, device="cuda", generator=g) * 0.2).clamp(-1, 1)
+    out = {}
+    for kernel in ("tensor", "tensor_unswizzled", "cuda"):
+        ops.set_fxp_kernel(kernel)
+        try:
+            out[kernel] = ops.conv2d_saturate_acc(x, wt, 0, 7, 24, (k // 2, k // 2), (1, 1))
+            assert ops.workspace_status() == 0
+        finally:
+            ops.set_fxp_kernel("auto")
+    assert torch.equal(out["tensor"], out["cuda"]) and torch.equal(out["tensor_unswizzled"], out["cuda"])
