@@ -104,10 +104,24 @@ static int conv_expand(const rexsc_sc_conv_desc *desc, const void *d_act, const 
     if (k == REXSC_KERNEL_TENSOR && d_act) {
         // one launch for the whole stage (it also clears the status block) where the shape qualifies
         const bool no_w = d_weight == nullptr;
+        // not while an operand is still to be read from the same memory (an output on the activation's storage)
+        auto clear_words = [&](const ConvPlan &plan) -> long long {
+            if (!outputs_cleared) return 0;
+            const size_t out_bytes = (size_t)plan.M * plan.Co * sizeof(int16_t);
+            auto overlap = [&](const void *out, const void *in, long long n, int dtype) {
+                const uintptr_t o = reinterpret_cast<uintptr_t>(out), i = reinterpret_cast<uintptr_t>(in);
+                return o < i + (size_t)n * (dtype == REXSC_F32 ? 4 : 2) && i < o + out_bytes;
+            };
+            for (const int16_t *out : {d_out_pos, d_out_neg})
+                if (overlap(out, d_act, (long long)plan.N * plan.C * plan.H * plan.W, desc->act_dtype) ||
+                    overlap(out, d_weight, plan.Kdot * plan.Co, desc->w_dtype))
+                    return 0;
+            return conv_tc_clear_words(plan, *desc, d_out_pos, d_out_neg);
+        };
         if (mode == kGridSpeculative) {
             REXSC_CUDA_CHECK(cudaMemsetAsync(b.status, 0, 256, st));
             // (cleared for the launch on the compact grid; the one on the standard grid stores whole tiles)
-            const long long clear = outputs_cleared ? conv_tc_clear_words(pc, *desc, d_out_pos, d_out_neg) : 0;
+            const long long clear = clear_words(pc);
             rc = launch_expand_all_bits(pc, *desc, d_act, d_weight, xnor, Ab, Wb, b.status,
                                         ExpandAllOptions{true, false, no_w, {d_out_pos, d_out_neg}, clear}, st);
             if (rc == REXSC_OK && clear > 0) *outputs_cleared = true;
@@ -115,7 +129,7 @@ static int conv_expand(const rexsc_sc_conv_desc *desc, const void *d_act, const 
                 rc = launch_expand_all_bits(p, *desc, d_act, d_weight, xnor, Ab, Wb, b.status,
                                             ExpandAllOptions{false, true, true, {nullptr, nullptr}, 0}, st);
         } else {
-            const long long clear = outputs_cleared ? conv_tc_clear_words(pa, *desc, d_out_pos, d_out_neg) : 0;
+            const long long clear = clear_words(pa);
             rc = launch_expand_all_bits(pa, *desc, d_act, d_weight, xnor, Ab, Wb, b.status,
                                         ExpandAllOptions{false, false, no_w, {d_out_pos, d_out_neg}, clear}, st);
             if (rc == REXSC_OK && clear > 0) *outputs_cleared = true;

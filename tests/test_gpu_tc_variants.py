@@ -65,3 +65,23 @@ def test_caller_padded_layers(ops, n, c, co, border):
     """A zero border (compact grid) and one that is not (found out by the expand launch)."""
     _both(ops, n, c, 7, 7, co, 3, 1, 1, False, 32, 2, True, torch.float16, border)
     _both(ops, n, c, 7, 7, co, 3, 1, 1, False, 32, 2, False, torch.float32, border)
+
+
+@pytest.mark.parametrize("on", ["input", "weight"])
+def test_output_on_an_operands_storage(ops, on):
+    """``out`` tensors that share the activation's or the weight's memory: both are read before an output is written,
+    although the outputs of so small a layer are cleared by the launch that reads the operands."""
+    g = torch.Generator(device="cuda").manual_seed(5)
+    h = 56 if on == "input" else 3
+    fmt = torch.channels_last
+    x = (torch.randn(1, 64, h, h, device="cuda", generator=g) * 0.45).clamp(0, 1).half().contiguous(memory_format=fmt)
+    wt = (torch.randn(64, 64, 3, 3, device="cuda", generator=g) * 0.2).clamp(-1, 1).half().contiguous(memory_format=fmt)
+    args = (32, -1, 16, (1, 1), (1, 1), (7, 8, 1), 1, 1, True, False)
+    want = ops.conv2d_generic_general_split_acc(x, wt, *args)
+    if on == "input":
+        shared = x.view(torch.int16)
+    else:
+        shared = wt.permute(0, 2, 3, 1).reshape(-1)[:64 * h * h].view(torch.int16).view(1, h, h, 64).permute(0, 3, 1, 2)
+        assert shared.data_ptr() == wt.data_ptr()
+    got = ops.conv2d_generic_general_split_acc(x, wt, *args, out=(shared, torch.empty_like(shared)))
+    assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
