@@ -4,6 +4,8 @@ direct kernel, which the oracle tests cover."""
 import pytest
 import torch
 
+from test_gpu_sc_conv import _torch_loop_linear_counts
+
 pytestmark = pytest.mark.gpu
 
 
@@ -85,3 +87,90 @@ def test_output_on_an_operands_storage(ops, on):
         assert shared.data_ptr() == wt.data_ptr()
     got = ops.conv2d_generic_general_split_acc(x, wt, *args, out=(shared, torch.empty_like(shared)))
     assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+
+
+@pytest.mark.parametrize("lfsr", [1, 2])
+@pytest.mark.parametrize("xnor", [True, False])
+@pytest.mark.parametrize("nhwc", [True, False])
+def test_shortest_registers(ops, oracle, lfsr, xnor, nhwc):
+    """Explicit 1- and 2-bit registers, whose cycle is one state longer than the 2^l - 1 of the others, on the merged
+    expand launch (32 and 64 slots) and the separate ones (128)."""
+    g = torch.Generator().manual_seed(lfsr)
+    x = torch.rand(2, 40, 7, 9, generator=g)
+    wt = (torch.randn(70, 40, 3, 3, generator=g) * 0.5).clamp(-1, 1)
+    if nhwc:
+        x, wt = x.contiguous(memory_format=torch.channels_last), wt.contiguous(memory_format=torch.channels_last)
+    for L in (32, 64, 128):
+        args = (L, lfsr, 16, (1, 1), (1, 1), (7, 8, 1), 1, 1, xnor, False)
+        want = oracle.conv2d_generic_general_split(x, wt, *args)
+        assert int(want[0].sum()) > 0
+        for kernel in ("tensor", "direct"):
+            ops.set_conv_kernel(kernel)
+            try:
+                got = ops.conv2d_generic_general_split_acc(x.cuda(), wt.cuda(), *args)
+            finally:
+                ops.set_conv_kernel("auto")
+            assert torch.equal(got[0].cpu(), want[0]) and torch.equal(got[1].cpu(), want[1]), (kernel, L)
+
+
+@pytest.mark.parametrize("c,k,low,co", [(2016, 1, 0.9, 64), (227, 3, 0.9, 70), (504, 2, 0.9, 64),   # every count is summed as it is
+                                        (8191, 1, 0.3, 64), (910, 3, 0.3, 64), (2047, 2, 0.3, 70)])  # counts around the limit
+@pytest.mark.parametrize("nhwc", [True, False])
+def test_counts_in_the_thousands(ops, c, k, low, co, nhwc):
+    """Dense operands, an output channel's weights of one sign, the largest n: fp32 accumulators have to hold integers
+    of this size exactly on top of their 2^23."""
+    g = torch.Generator(device="cuda").manual_seed(c)
+    x = torch.rand(2, c, 5, 7, device="cuda", generator=g) * (1 - low) + low
+    wt = torch.rand(co, c, k, k, device="cuda", generator=g) * (1 - low) + low
+    wt[1::2] *= -1
+    fmt = torch.channels_last if nhwc else torch.contiguous_format
+    x, wt = x.contiguous(memory_format=fmt), wt.contiguous(memory_format=fmt)
+    out = []
+    for kernel in ("tensor", "direct"):
+        ops.set_conv_kernel(kernel)
+        try:
+            out.append(ops.conv2d_generic_general_split_acc(x, wt, 32, -1, 16, (0, 0), (1, 1), (7, 8, 1), 2046, 1, True, False))
+            assert ops.workspace_status() == 0
+        finally:
+            ops.set_conv_kernel("auto")
+    sums = [t.to(torch.int32) & 0xffff for t in out[1]]
+    assert sums[0][:, 0::2].float().mean() > 32 * 1500 and sums[1][:, 1::2].float().mean() > 32 * 1500
+    for a, b in zip(*out):
+        assert torch.equal(a, b), f"{(a != b).sum().item()} counts differ"
+
+
+@pytest.mark.parametrize("c,co,k", [(500, 300, 3), (402, 260, 3), (1000, 1030, 1)])
+@pytest.mark.parametrize("w_nhwc", [True, False])
+@pytest.mark.parametrize("w_dtype", [torch.float32, torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("L", [32, 64])
+def test_large_filters(ops, c, co, k, w_nhwc, w_dtype, L):
+    """Weights expanded in blocks of 32 output channels (512 blocks and more): channels that end inside a word, output
+    channels that end inside a block, vector and scalar loads, one and two words per stream."""
+    g = torch.Generator(device="cuda").manual_seed(c + co)
+    x = (torch.randn(1, c, 5, 6, device="cuda", generator=g) * 0.45).clamp(0, 1)
+    wt = (torch.randn(co, c, k, k, device="cuda", generator=g) * 0.2).clamp(-1, 1).to(w_dtype)
+    wt[0, :, 0, 0] = float("nan")
+    wt = wt.contiguous(memory_format=torch.channels_last if w_nhwc else torch.contiguous_format)
+    p = k // 2
+    out = []
+    for kernel in ("tensor", "direct"):
+        ops.set_conv_kernel(kernel)
+        try:
+            out.append(ops.conv2d_generic_general_split_acc(x, wt, L, -1, 16, (p, p), (1, 1), (7, 8, 1), 2, 1, True, False))
+        finally:
+            ops.set_conv_kernel("auto")
+    for a, b in zip(*out):
+        assert torch.equal(a, b), f"{(a != b).sum().item()} counts differ"
+
+
+@pytest.mark.parametrize("L", [32, 64])
+@pytest.mark.parametrize("c,co", [(1000, 1000), (998, 1030)])
+def test_large_linear_layer_with_seeds_of_its_own(ops, L, c, co):
+    """The same blocks with linear seeds, other offsets for positive than for negative weights."""
+    g = torch.Generator().manual_seed(c)
+    top = (L - 1) / L
+    x = ((torch.rand(3, c, generator=g) * 128).floor() / 128).clamp(max=top)
+    wt = ((torch.randn(co, c, generator=g) * 0.2).clamp(-1, 1) * 128).round().div(128).clamp(-top, top)
+    want = _torch_loop_linear_counts(x.numpy(), wt.numpy(), L, (67, 37), True)
+    got = ops.linear_generic_general_acc(x.cuda(), wt.cuda(), (7, 8, 1), L, -1, 0, 1, False, False, weight_seeds=(67, 37))
+    assert all((t.cpu().numpy() == w).all() for t, w in zip(got, want))
