@@ -44,7 +44,6 @@
 // Every wait is bounded; on a time-out the CTA reports through the status word, frees its TMEM and returns.
 #include "common.cuh"
 #include <stdlib.h>
-#include <type_traits>
 
 namespace rexsc {
 
@@ -88,8 +87,7 @@ constexpr uint32_t kTcSuspendNs = 4000;    // a waiting warp sleeps in the barri
 
 struct TcArgs {
     int OH, OW, KHW, Co, CW;
-    int KWc;         // 32-channel words per pipeline step (even: one MMA takes two)
-    int CK;          // pipeline steps per slot = ceil(CW / KWc)
+    int CK;          // pipeline steps per slot = ceil(CW / KWC)
     int depth;       // steps of bit words kept in shared memory: kTcMaxDepth, or 2 when it is short
     int nrh, nrw, Wq, Hrows, Wrow; // stored pixel grid (see tap_offset in common.cuh)
     int Ho, Wo;      // origin grid of one image
@@ -222,7 +220,7 @@ __device__ __forceinline__ uint4 spread_weights(uint32_t h)
         :: "memory")
 
 // KHW_T: taps known at compile time (9, 1) or 0 for any tap count up to kTcMaxTaps
-// KWC:   32-channel words per pipeline step (TcArgs::KWc; above 4 only with KHW_T == 1)
+// KWC:   32-channel words per pipeline step (even: one MMA takes two; above 4 only with KHW_T == 1)
 // RA:    patch rows per expanding thread (1 .. kTcMaxARows)
 //
 // What bounds it, and the split of the warps.  The MMAs of a step take 18 x 83 clk on a 3x3 layer; everything else has
@@ -473,7 +471,7 @@ sc_conv_tc_kernel(TcArgs a, const uint32_t *__restrict__ Ab, const uint32_t *__r
         const int my_tiles = run.tiles;
         const uint32_t *a_plane = Ab;
         uint32_t a_off[RA]; // stored-grid position of the thread's patch rows, ~0u: outside the tensor
-        int ld_ck = 0, ld_left = 0, ld_tile = -1, ld_d = 0, ld_round = 0;
+        int ld_ck = 0, ld_left = 0, ld_tile = -1, ld_d = 0;
         // point the loads at the first slot and chunk of tile k of this CTA
         auto load_tile = [&](int k) {
             long long o0;
@@ -524,7 +522,7 @@ sc_conv_tc_kernel(TcArgs a, const uint32_t *__restrict__ Ab, const uint32_t *__r
                     a_plane += (size_t)KWC * a.NHWp;
                 }
                 if (--ld_left == 0 && ld_tile + 1 < my_tiles) load_tile(ld_tile + 1); // the next call fetches the next tile
-                ring_next(ld_d, ld_round);
+                if (++ld_d == a.depth) ld_d = 0;
             }
             asm volatile("cp.async.commit_group;" ::: "memory");
         };
@@ -906,8 +904,9 @@ bool conv_tc_supported(const ConvPlan &p)
     if (!g.ok) return false;
     const long long cap = p.n_or < p.Kdot ? p.n_or : p.Kdot;                   // largest per-slot contribution
     if ((long long)p.words * 32 * cap > 65535) return false;                  // 16-bit running sums
-    if (p.Kdot > 8191) return false;                                          // (far below what fp32 counts exactly)
-    if (p.Kdot > (1 << 24)) return false;
+    // The packed read of 2^23 + count has room for counts up to 65535.  Longer dot products than 8191 have not been run on
+    // this path and stay where they are, on the ALU kernels.
+    if (p.Kdot > 8191) return false;
     const long long total_o = (long long)p.N * g.Ho * g.Wo;
     if (total_o + kTcM > 0x7fffffffLL) return false;                          // 31-bit candidate indices
     if ((total_o + kTcM - 1) / kTcM * ((p.Co + kTcCout - 1) / kTcCout) > 0x7fffffffLL) return false; // tile index: int
@@ -1000,7 +999,7 @@ int launch_conv_tc(const ConvPlan &p, const rexsc_sc_conv_desc &d, void *d_tc_ws
     const uint32_t *Wb = reinterpret_cast<const uint32_t *>(static_cast<const uint8_t *>(d_tc_ws) + weight_offset);
     TcArgs a;
     a.OH = p.OH; a.OW = p.OW; a.KHW = p.KHW; a.Co = p.Co;
-    a.CW = CW; a.KWc = g.KWc; a.CK = g.CK; a.depth = g.depth;
+    a.CW = CW; a.CK = g.CK; a.depth = g.depth;
     a.nrh = p.nrh; a.nrw = p.nrw; a.Wq = p.Wq; a.Hrows = p.Hrows; a.Wrow = p.Wrow;
     a.Ho = g.Ho; a.Wo = g.Wo; a.Mh = g.Mh; a.rows_a = g.rows_a;
     a.shift = p.origin ? g.Wo + 1 : 0;

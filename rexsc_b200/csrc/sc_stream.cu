@@ -1103,9 +1103,8 @@ struct ExpandWBitsArgs {
 // ---- the whole expand stage of a tensor-core conv call in ONE launch ------------------------------------------------
 // Stream tables, weight bit planes and activation bit planes used to be three dependent launches (plus the clearing of
 // the status word); for the smaller layers their launch latencies, not their work, made up most of the stage.  Here
-// every CTA builds both tables in its own shared memory straight from the LFSR (a few thousand short generator runs
-// per CTA, nothing read from global memory), takes its share of the weight items, then runs the pipelined activation
-// expansion.
+// every CTA builds the table of both operands in its own shared memory from the tabulated cycle of the register, takes its
+// share of the weight items, then runs the pipelined activation expansion.
 // Table of stream words of every (seed phase, value), built in shared memory without running the generator.
 // Valid for gen_config 1 with progressive loading inactive (the front end's settings), where the activation and the
 // weight table coincide.  The generator seeded with state s emits at step t the comparison value > orbit[pos(s) + t + 1],
@@ -1179,6 +1178,11 @@ __device__ __forceinline__ float load_weight_any(const void *w, int dtype, long 
     if (dtype == REXSC_F16) return __half2float(static_cast<const __half *>(w)[i]);
     return __bfloat162float(static_cast<const __nv_bfloat16 *>(w)[i]);
 }
+
+// Shared-memory staging of a warp: two activation tiles of 32 pixels x 32 channels, 4 bytes each for every type.  (Half of
+// it for the 2-byte types lets a second CTA beside the 64-slot table: 64 x 64 channels 56x56 NCHW 126 -> 81 us, but
+// 8 x 256 channels 14x14 37 -> 41 us.)
+constexpr int kAllStaging = 2 * 32 * 32 * 4;
 
 template <typename T, int WORDS, bool NCHW>
 __global__ void __launch_bounds__(kFastWarps * 32, 2)
@@ -1296,7 +1300,9 @@ expand_all_kernel(ExpandAllArgs g, const T *__restrict__ x, const void *__restri
         // Large filters: 32 output channels x 32 input channels of one tap per item, lane = output channel.  A lane looks
         // the stream words of its 32 input channels up (their seed phases are the same in all lanes), transposes them in
         // its registers like the activation path, and every slot's words leave as one 128-byte run.  Input channel c goes
-        // to row (c with its low two bits reversed), which leaves the nibbles of the slot words bit-reversed.
+        // to row (c with its low two bits inverted), which leaves the nibbles of the slot words bit-reversed.
+        // (With two words per stream ptxas keeps 240-340 bytes of this part's state in local memory, at the 128 registers that
+        // two CTAs per SM leave; the stage as a whole is no slower for it than with the shared-memory tiles before.)
         for (long long item = (long long)blockIdx.x * kFastWarps + warp; g.w_coarse && item < g.w_items;
              item += (long long)gridDim.x * kFastWarps) {
             const int cw = (int)(item % wa.CW);
@@ -1360,7 +1366,7 @@ expand_all_kernel(ExpandAllArgs g, const T *__restrict__ x, const void *__restri
         }
     }
     // (each warp goes on as soon as its own weight items are done: its staging area is its own)
-    expand_act_async_body<T, WORDS, NCHW>(a, x, lut_s, reinterpret_cast<uint8_t *>(lut_s) + lut_smem_bytes, 8192, sh, Ab, CW, n_groups, g.cw_parts);
+    expand_act_async_body<T, WORDS, NCHW>(a, x, lut_s, reinterpret_cast<uint8_t *>(lut_s) + lut_smem_bytes, kAllStaging, sh, Ab, CW, n_groups, g.cw_parts);
 }
 
 template <typename T, int WORDS, bool NCHW>
@@ -1382,9 +1388,7 @@ static int launch_expand_all_t(ExpandAllArgs g, const void *d_act, const void *d
     if (blocks < wblocks) blocks = wblocks;
     if (blocks > 2LL * sms) blocks = 2LL * sms; // persistent: two CTAs per SM
     const size_t lut_al = (lut_bytes + 15) / 16 * 16;
-    // per warp: two activation tiles of 32 pixels x 32 channels, and at least the two 4 KB weight tiles
-    const size_t staging = (size_t)kFastWarps * 8192;
-    static_assert(2 * 32 * 32 * sizeof(T) <= 8192, "activation staging exceeds the per-warp area");
+    const size_t staging = (size_t)kFastWarps * kAllStaging;
     auto kernel = expand_all_kernel<T, WORDS, NCHW>;
     REXSC_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(lut_al + staging)));
     kernel<<<(unsigned)blocks, kFastWarps * 32, lut_al + staging, st>>>(g, (const T *)d_act, d_w, d_Ab, d_Wb, d_status, CW,
