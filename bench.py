@@ -20,8 +20,8 @@ One JSON line is printed by rank 0:
              them under autocast; `e2e_fp32_activations` repeats it with fp32 activations); --e2e-slots / --e2e-chunks
              set the staging depth and the batch slicing of the host pipeline
   gpu_launches  this library's kernels inside the timed region, as the library counts them
-  roofline   dominant kernel: the tensor-core SC conv (one 4-bit tcgen05 GEMM per time slot) against the 4-bit tensor
-             rate measured live by a back-to-back MMA probe; `roofline_secondary` / `roofline_expand` the ALU kernel
+  roofline   dominant kernel: the tensor-core SC conv (one 4-bit tcgen05 GEMM per time slot) against twice the int8 tensor
+             rate, which is measured live by a back-to-back MMA probe; `roofline_secondary` / `roofline_expand` the ALU kernel
              and the stream-expansion stage; `roofline_pointwise` the four point-wise kernels against HBM
   train      images/s of full training steps (fwd + bwd + optimizer) of the reference's own model and loop on the
              drop-in ops, per `sync` mode, with the NCCL weight-gradient all-reduce when N > 1
@@ -472,17 +472,18 @@ def sc_line(args, wl, r, world):
     alu_achieved = a["lop3"] / (a["ms"] * 1e-3) if a["ms"] > 0 else 0.0
     roof_tensor = {
         "bound": "tensor", "kernel": "sc_conv_tc_kernel (tcgen05 mxf4, one GEMM per time slot)",
-        # the 4-bit kind takes K = 64 in the clocks that int8 takes K = 32 (both 67 clk for M128 N128): twice the probe rate
+        # no 4-bit probe: the 4-bit kind takes K = 64 in the clocks that int8 takes K = 32 (both measured at 67 clk for M128
+        # N128), so the rate is taken as twice that of the int8 probe
         "achieved": tc_achieved / 1e12, "peak": 2 * r["mma_peak_ops"] / 1e12, "unit": "TOP/s 4-bit",
         "frac": tc_achieved / (2 * r["mma_peak_ops"]),
-        # per average launch: reads = 1.23 x the activation bit planes, the ratio of ncu's dram__bytes_read.sum
-        # (65.6 MB) to the planes (53.2 MB) of the captured 64-channel layer at batch 64 (patch halos, the
+        # per average launch: reads = 1.31 x the activation bit planes, the ratio of ncu's dram__bytes_read.sum
+        # (72.3 MB) to the planes (55.1 MB) of the captured 64-channel layer at batch 64 (patch halos, the
         # read-modify-write of cut tiles and the weight planes make up the rest; it grows in proportion to the batch);
-        # writes = the int16 outputs (a single captured launch leaves most of them in L2 -- 13.0 of 51.4 MB had been
+        # writes = the int16 outputs (a single captured launch leaves most of them in L2 -- 16.7 of 51.4 MB had been
         # written back when the capture ended -- a whole step, whose layers do not fit L2 together, writes them all)
-        "traffic": ((0.23 * t["plane_bytes"] + t["bytes"]) / t["launches"]) if t["launches"] else None,
+        "traffic": ((0.31 * t["plane_bytes"] + t["bytes"]) / t["launches"]) if t["launches"] else None,
         "traffic_source": "ncu capture of one layer at batch 64 (read ratio), scaled by algorithmic bytes",
-        "peak_source": "measured live: back-to-back tcgen05.mma kind::i8 M128 N128 K32 probe on this GPU",
+        "peak_source": "2 x the rate of a back-to-back tcgen05.mma kind::i8 M128 N128 K32 probe, measured live on this GPU",
         "kernel_ms_per_step": t["ms"], "launches_per_step": t["launches"],
         "tbitops_per_s_kernel": t["intops"] / 2 / (t["ms"] * 1e-3) / 1e12 if t["ms"] > 0 else 0.0,
     }
