@@ -25,8 +25,10 @@ One JSON line is printed by rank 0:
              and the stream-expansion stage; `roofline_pointwise` the four point-wise kernels against HBM
   train      images/s of full training steps (fwd + bwd + optimizer) of the reference's own model and loop on the
              drop-in ops, per `sync` mode, with the NCCL weight-gradient all-reduce when N > 1
-  cpu_baseline  the reference's own CPU extension (oracle/_ref) on a bounded sample, N=1 only
-`--impl reference` times that CPU extension alone (all host threads) on the same layer list at a reduced batch.
+  cpu_baseline  the reference's own CPU extension (oracle/_ref) on a bounded sample, N=1 only (`kind` "port": the
+             oracle's restatement of it, where the extension does not run)
+`--impl reference` times that CPU extension alone (all host threads) on the same layer list at a reduced batch, or says
+`unavailable` where it is not built or does not run.
 """
 from __future__ import annotations
 
@@ -802,13 +804,14 @@ def run_reference(args, wl, rank, world):
     threads = os.cpu_count() or 1
     os.environ.setdefault("OMP_NUM_THREADS", str(threads))
     sb = _sample_batch(wl)
-    load_reference_cpu()
+    if load_reference_cpu() is None:  # the oracle port is this project's code: it does not stand in for the reference
+        return {"impl": "reference", "unavailable": "the reference's CPU extensions are not built here (oracle/_ref) or do "
+                                                    "not run on this host"}
     if args.warmup > 0:
         cpu_reference_time(dict(wl, layers=wl["layers"][-1:]), sb, threads)
     t0 = time.perf_counter()
-    kind = "reference"
     for _ in range(args.steps):
-        _, kind = cpu_reference_time(wl, sb, threads)
+        cpu_reference_time(wl, sb, threads)
     dt = time.perf_counter() - t0
     value = sb * args.steps / dt
     unit = "rows/s" if wl["kind"] == "linear" else "img/s"
@@ -820,7 +823,7 @@ def run_reference(args, wl, rank, world):
         "data": "synthetic",
         # the same workload description as the other arm; what a step samples of it is in cpu_baseline.sample
         "config": {"workload": wl["text"], "batch_per_gpu": wl["batch"]},
-        "cpu_baseline": {"value": value, "unit": unit, "cores": threads, "kind": kind, "sample": sample},
+        "cpu_baseline": {"value": value, "unit": unit, "cores": threads, "kind": "reference", "sample": sample},
         "e2e": {"value": value, "unit": unit, "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0},
         "gpu_launches": 0,
     }

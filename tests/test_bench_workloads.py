@@ -31,3 +31,14 @@ def test_workload_layer_lists_and_bit_op_totals():
         assert wl["metric"] and wl["batch"] >= 1 and wl["text"]
         assert 1 <= bench._sample_batch(wl) <= wl["batch"] or wl["kind"] == "linear"
     assert bench._sample_batch(w["resnet18"]) == 4
+
+
+def test_reference_arm_without_the_reference(monkeypatch):
+    """No code of this project stands in for the reference's: the arm says that it is unavailable."""
+    import argparse
+
+    import bench
+
+    monkeypatch.setitem(bench._REF_CPU, "mods", None)
+    line = bench.run_reference(argparse.Namespace(gpus=1, steps=1, warmup=0), bench.WORKLOADS["conv5x5"], 0, 1)
+    assert line["impl"] == "reference" and line["unavailable"] and "value" not in line
