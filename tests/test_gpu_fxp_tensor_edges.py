@@ -27,11 +27,13 @@ def test_tensor_kernel_equals_cuda_kernel(ops, n, c, h, w, co, k, pad, dtype):
 
 @pytest.mark.parametrize("c,k", [(4, 1), (16, 1), (17, 1), (33, 1), (59, 1), (64, 1), (65, 1), (128, 1), (130, 1), (160, 1),
                                  (176, 1), (15, 3), (33, 3), (50, 2)])
-@pytest.mark.parametrize("co", [10, 83, 300])
-def test_blocks_of_a_last_slab(ops, c, k, co):
-    """One step and several; last slabs of one, two, three and four blocks of 32 products; one to three channel chunks."""
+@pytest.mark.parametrize("n,h,w,co", [(3, 9, 12, 10), (3, 9, 12, 83), (3, 9, 12, 300),
+                                      (19, 32, 32, 10), (19, 32, 32, 300)])
+def test_blocks_of_a_last_slab(ops, n, h, w, co, c, k):
+    """One step and several; last slabs of one, two, three and four blocks of 32 products; one to three channel chunks;
+    fewer CTAs than SMs (two weight buffers) and more (one)."""
     g = torch.Generator(device="cuda").manual_seed(c * 1000 + co)
-    x = torch.rand(3, c, 9, 12, device="cuda", generator=g)
+    x = torch.rand(n, c, h, w, device="cuda", generator=g)
     wt = (torch.randn(co, c, k, k, device="cuda", generator=g) * 0.2).clamp(-1, 1)
     out = {}
     for kernel in ("tensor", "tensor_unswizzled", "cuda"):
